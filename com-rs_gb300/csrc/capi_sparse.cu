@@ -46,6 +46,8 @@ struct cb_ldpc {
   bool regs = false;     // layered sum-product rows in registers
   bool has_aux = true;   // a second message buffer
   int group = 1;         // codewords per CTA
+  int chain_group = 0;   // chained rows (sparse_chain.cu): slots per row, 0 for the other kernels
+  cbk::ChainDev chain{};
   void* kernel = nullptr;
   cudaStream_t stream = nullptr;
   void* d_llr = nullptr;
@@ -92,7 +94,6 @@ cudaError_t grow_buf(void** ptr, size_t& cap, size_t bytes) {
 
 size_t elem(const cb_ldpc* c) { return c->precision == CB_F64 ? 8 : 4; }
 
-// device tables, launch shape and message storage, on first use
 cb_status ensure_stream(cb_ldpc* c) {
   LDPC_CUDA(c, cudaSetDevice(c->device));
   if (!c->stream) LDPC_CUDA(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
@@ -114,10 +115,70 @@ void release_decoder(cb_ldpc* c) {
   c->dev_ready = false;
 }
 
+// The chained decoder (sparse_chain.cu) for a layered code of one-row levels whose rows
+// form blocks of 16 or more on average: its results are the warp-per-row path's, whose
+// latency it cuts (DVB-S2 short rate 1/2, f32 sum-product, 152 words: 65 ms with a warp
+// per row, 4.5 ms in blocks of 64 rows).  A block costs about 3.5 us whatever its rows (a
+// start and an end of 1.5 us, ten chain sweeps), a row on a warp of its own 0.8 us, so
+// blocks pay from some five rows on; 16 leaves room for chains that take more sweeps.
+bool use_chain(const cb_ldpc* c, const cbh::ChainBlocks& blocks) {
+  const cbh::SparseCode& h = c->host;
+  return (int64_t)h.m >= 16 * (int64_t)(blocks.block_start.size() - 1);
+}
+
+cb_status ensure_chain(cb_ldpc* c, const cbh::ChainBlocks& blocks) {
+  const cbh::SparseCode& h = c->host;
+  const int g = h.max_row_degree <= 8 ? 8 : h.max_row_degree <= 16 ? 16 : 32;
+  std::vector<int32_t> info(h.m), vars((size_t)h.m * g, -1);
+  for (int r = 0; r < h.m; r++) {
+    const int d = h.row_start[r + 1] - h.row_start[r];
+    info[r] = d | (blocks.linked[r] ? (int)cbk::kChainLinkIn : 0) |
+              (r + 1 < h.m && blocks.linked[r + 1] ? (int)cbk::kChainLinkOut : 0);
+    for (int k = 0; k < d; k++) vars[(size_t)r * g + k] = h.vars[h.row_start[r] + k];
+  }
+  const std::vector<int32_t>& bs = blocks.block_start;
+  LDPC_CUDA(c, cudaMalloc(&c->d_tables, (bs.size() + info.size() + vars.size()) * 4));
+  int32_t* p = c->d_tables;
+  cbk::ChainDev& d = c->chain;
+  d.n = h.n;
+  d.m = h.m;
+  d.blocks = (int32_t)bs.size() - 1;
+  d.block_start = p;
+  d.row_info = p + bs.size();
+  d.vars = p + bs.size() + info.size();
+  LDPC_CUDA(c, cudaMemcpy(p, bs.data(), bs.size() * 4, cudaMemcpyHostToDevice));
+  LDPC_CUDA(c, cudaMemcpy(p + bs.size(), info.data(), info.size() * 4, cudaMemcpyHostToDevice));
+  LDPC_CUDA(c, cudaMemcpy(p + bs.size() + info.size(), vars.data(), vars.size() * 4, cudaMemcpyHostToDevice));
+  LDPC_CUDA(c, cudaMalloc(&c->d_counter, sizeof(unsigned long long)));
+  const size_t post_bytes = (size_t)h.n * elem(c);
+  c->post_in_smem = post_bytes <= kSmemPostBudget;
+  c->smem = c->post_in_smem ? ((post_bytes + 15) & ~(size_t)15) : 0;
+  c->threads = cbk::sparse_chain_threads(g);
+  c->group = 1;
+  c->kernel = cbk::sparse_chain_kernel_ptr(c->precision == CB_F64 ? 0 : 1, c->rule, g);
+  LDPC_CUDA(c, cudaFuncSetAttribute(c->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->smem));
+  int per_sm = 0, sms = 0;
+  LDPC_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, c->kernel, c->threads, c->smem));
+  LDPC_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  const size_t slot_bytes = (size_t)h.m * g * elem(c) + (c->post_in_smem ? 0 : post_bytes);
+  c->grid = std::max(1, per_sm * sms);
+  c->grid = std::min<int>(c->grid, (int)std::max<size_t>(1, ((size_t)2 << 30) / slot_bytes));
+  LDPC_CUDA(c, cudaMalloc(&c->d_slots, (size_t)c->grid * slot_bytes));
+  c->chain_group = g;
+  c->dev_ready = true;
+  return CB_OK;
+}
+
+// device tables, launch shape and message storage, on first use
 cb_status ensure_device(cb_ldpc* c) {
   if (c->dev_ready) return CB_OK;
   const cbh::SparseCode& h = c->host;
   if (cb_status st = ensure_stream(c)) return st;
+  c->chain_group = 0;
+  if (c->layered && h.max_level_rows == 1 && h.max_row_degree <= 32) {
+    const cbh::ChainBlocks blocks = cbh::chain_blocks(h, cbk::kChainBlockRows);
+    if (use_chain(c, blocks)) return ensure_chain(c, blocks);
+  }
   // the launch shape decides the message layout: a thread per row with messages in
   // global memory takes the transposed one
   c->warp_rows = c->layered && h.max_level_rows <= 8 && h.max_row_degree <= 128;
@@ -220,6 +281,24 @@ cb_status ensure_device(cb_ldpc* c) {
 template <typename T>
 cb_status decode_impl(cb_ldpc* c, const T* llr, int64_t n, T* post, int32_t* iters, cudaStream_t s) {
   if (n == 0) return CB_OK;
+  if (c->chain_group) {
+    cbk::ChainArgs<T> a;
+    a.code = c->chain;
+    a.alpha = c->alpha;
+    a.oms = c->rule == CB_RULE_OMS ? 1 : 0;
+    a.max_iterations = c->max_iterations;
+    a.post_in_smem = c->post_in_smem ? 1 : 0;
+    a.reserved = 0;
+    a.llr = llr;
+    a.n_frames = n;
+    a.post_out = post;
+    a.iters_out = iters;
+    a.slots = reinterpret_cast<T*>(c->d_slots);
+    a.work_counter = c->d_counter;
+    LDPC_CUDA(c, cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned long long), s));
+    LDPC_CUDA(c, cbk::launch_sparse(c->kernel, &a, (int)std::min<int64_t>(c->grid, n), c->threads, c->smem, s));
+    return CB_OK;
+  }
   cbk::SparseArgs<T> a;
   a.code = c->dev;
   a.alpha = c->alpha;

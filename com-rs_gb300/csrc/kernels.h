@@ -222,6 +222,33 @@ constexpr int kMaxGroup = 8;
 void* sparse_group_kernel_ptr(int precision, int rule, bool regs);
 cudaError_t launch_sparse(void* kernel, const void* args, int grid, int threads, size_t smem, cudaStream_t stream);
 
+// ---- layered decoding of chained rows (sparse_chain.cu): blocks of consecutive rows
+// whose variables are distinct, but for the last variable of a row and the second to last
+// of the next.  A row's edges take `group` (8, 16 or 32) slots.
+constexpr int kChainBlockRows = 64;
+constexpr uint32_t kChainLinkIn = 64;    // row_info: the second to last variable comes from the row before
+constexpr uint32_t kChainLinkOut = 128;  // row_info: the next row takes the last variable over
+struct ChainDev {
+  int32_t n, m, blocks;
+  const int32_t* block_start;  // blocks + 1
+  const int32_t* row_info;     // m: the degree (bits 0-5) and the link flags
+  const int32_t* vars;         // m x group, -1 beyond a row's degree
+};
+template <typename T>
+struct ChainArgs {
+  ChainDev code;
+  double alpha;
+  int32_t oms, max_iterations, post_in_smem, reserved;
+  const T* llr;
+  int64_t n_frames;
+  T* post_out;
+  int32_t* iters_out;
+  T* slots;  // [grid][m group (+ n when !post_in_smem)]
+  unsigned long long* work_counter;
+};
+int sparse_chain_threads(int group);
+void* sparse_chain_kernel_ptr(int precision, int rule, int group);
+
 // ---- systematic encoders of generic codes (sparse_encode.cu)
 struct SumsEncodeArgs {
   const uint8_t* info;      // [n_frames][k]

@@ -83,6 +83,34 @@ bool build_sparse_code(int n, int m, const int32_t* row_start, const int32_t* va
   return true;
 }
 
+ChainBlocks chain_blocks(const SparseCode& c, int max_rows) {
+  ChainBlocks out;
+  out.linked.assign(c.m, 0);
+  std::vector<int> owner(c.n, -1);  // the last block that a variable was seen in
+  int block = -1, rows = 0;
+  for (int r = 0; r < c.m; r++) {
+    const int e0 = c.row_start[r], e1 = c.row_start[r + 1];
+    bool link = false, fits = block >= 0 && rows < max_rows;
+    for (int e = e0; e < e1 && fits; e++) {
+      if (owner[c.vars[e]] != block) continue;
+      // a variable of the block: only the link from the row before is allowed
+      if (e == e1 - 2 && c.row_start[r] > c.row_start[r - 1] && c.vars[e] == c.vars[e0 - 1]) link = true;
+      else fits = false;
+    }
+    if (!fits) {
+      out.block_start.push_back(r);
+      block++;
+      rows = 0;
+      link = false;
+    }
+    out.linked[r] = link;
+    for (int e = e0; e < e1; e++) owner[c.vars[e]] = block;
+    rows++;
+  }
+  out.block_start.push_back(c.m);
+  return out;
+}
+
 bool reduce_sums(const SparseCode& code, SparseEncoder& out, std::string& err) {
   const int n = code.n, m = code.m;
   const size_t words = (size_t)(n + 63) / 64;

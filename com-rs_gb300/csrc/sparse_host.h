@@ -34,6 +34,15 @@ struct SparseCode {
 bool build_sparse_code(int n, int m, const int32_t* row_start, const int32_t* vars, SparseCode& out,
                        std::string& err);
 
+// Consecutive rows in blocks of at most max_rows: a row joins the block of the row before
+// it when it shares no variable with the block's rows, except that its second to last
+// variable may be the last one of the row before (a link: the accumulator of an IRA code).
+struct ChainBlocks {
+  std::vector<int32_t> block_start;  // blocks + 1
+  std::vector<uint8_t> linked;       // m: the row is linked to the row before it
+};
+ChainBlocks chain_blocks(const SparseCode& code, int max_rows);
+
 // The systematic encoder of a code: the information positions and how the parity bits
 // follow from the information bits.
 enum EncoderKind { kEncoderNone = -1, kEncoderSums = 0, kEncoderAccumulate = 1 };
