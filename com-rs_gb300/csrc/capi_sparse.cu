@@ -25,6 +25,8 @@ constexpr size_t kSmemMsgBudget = 100 * 1024;
 constexpr size_t kSmemPostBudget = 200 * 1024;
 // shared memory of a CTA of several small codewords: two CTAs per SM
 constexpr size_t kGroupSmem = 100 * 1024;
+// shared memory of the edge-parallel sum-product decoder: one CTA per SM
+constexpr size_t kEdgeSmem = 224 * 1024;
 
 }  // namespace
 
@@ -48,6 +50,8 @@ struct cb_ldpc {
   int group = 1;         // codewords per CTA
   int chain_group = 0;   // chained rows (sparse_chain.cu): slots per row, 0 for the other kernels
   cbk::ChainDev chain{};
+  int edge_slots = 0;    // an edge per thread (sparse_edges.cu): codewords per CTA, 0 for the other kernels
+  cbk::EdgeDev edge{};
   void* kernel = nullptr;
   cudaStream_t stream = nullptr;
   void* d_llr = nullptr;
@@ -169,6 +173,43 @@ cb_status ensure_chain(cb_ldpc* c, const cbh::ChainBlocks& blocks) {
   return CB_OK;
 }
 
+// The edge-parallel sum-product decoder (sparse_edges.cu): `slots` codewords per CTA, one
+// CTA per SM.
+cb_status ensure_edges(cb_ldpc* c, int max_level_edges, int slots, int warps) {
+  const cbh::SparseCode& h = c->host;
+  std::vector<int32_t> tab(h.edges), row(1, 0), level(1, 0);
+  for (int l = 0, e = 0; l < h.levels; l++) {
+    for (int i = h.level_start[l]; i < h.level_start[l + 1]; i++) {
+      const int r = h.level_rows[i], d = h.row_start[r + 1] - h.row_start[r];
+      for (int k = 0; k < d; k++, e++)
+        tab[e] = (int32_t)((uint32_t)h.vars[h.row_start[r] + k] | (uint32_t)k << 16 | (uint32_t)d << 24);
+      row.push_back(e);
+    }
+    level.push_back(e);
+  }
+  tab.insert(tab.end(), row.begin(), row.end());
+  tab.insert(tab.end(), level.begin(), level.end());
+  LDPC_CUDA(c, cudaMalloc(&c->d_tables, tab.size() * 4));
+  LDPC_CUDA(c, cudaMemcpy(c->d_tables, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice));
+  LDPC_CUDA(c, cudaMalloc(&c->d_counter, sizeof(unsigned long long)));
+  const int p = c->precision == CB_F64 ? 0 : 1;
+  cbk::EdgeDev& d = c->edge;
+  d.n = h.n;
+  d.m = h.m;
+  d.edges = h.edges;
+  d.levels = h.levels;
+  d.max_level_edges = max_level_edges;
+  d.warps = warps;
+  d.edge = reinterpret_cast<const uint32_t*>(c->d_tables);
+  d.row = c->d_tables + h.edges;
+  d.level = d.row + h.m + 1;
+  c->kernel = cbk::sparse_edges_kernel_ptr(p);
+  LDPC_CUDA(c, cudaDeviceGetAttribute(&c->grid, cudaDevAttrMultiProcessorCount, c->device));
+  c->edge_slots = slots;
+  c->dev_ready = true;
+  return CB_OK;
+}
+
 // device tables, launch shape and message storage, on first use
 cb_status ensure_device(cb_ldpc* c) {
   if (c->dev_ready) return CB_OK;
@@ -178,6 +219,29 @@ cb_status ensure_device(cb_ldpc* c) {
   if (c->layered && h.max_level_rows == 1 && h.max_row_degree <= 32) {
     const cbh::ChainBlocks blocks = cbh::chain_blocks(h, cbk::kChainBlockRows);
     if (use_chain(c, blocks)) return ensure_chain(c, blocks);
+  }
+  // sum-product levels of more than eight rows whose word fits shared memory: an edge per
+  // thread, in f64 (1.8-3.7 times faster than a thread per row, sparse_edges.cu) and in f32
+  // (1.2-1.8 times).  Levels of fewer rows keep the warp per row, which associates the
+  // products as a scan does.
+  c->edge_slots = 0;
+  if (c->layered && c->rule == CB_RULE_SUM_PRODUCT && h.max_level_rows > 8) {
+    int max_level_edges = 0;
+    for (int l = 0; l < h.levels; l++) {
+      int e = 0;
+      for (int i = h.level_start[l]; i < h.level_start[l + 1]; i++)
+        e += h.row_start[h.level_rows[i] + 1] - h.row_start[h.level_rows[i]];
+      max_level_edges = std::max(max_level_edges, e);
+    }
+    const int p = c->precision == CB_F64 ? 0 : 1;
+    const size_t per = cbk::sparse_edges_slot_bytes(h.n, h.edges, max_level_edges, p);
+    const size_t tab = cbk::sparse_edges_table_bytes(h.edges, h.m, h.levels);
+    // a warp per 32 edges of the mean level
+    const int warps = std::min(cbk::kEdgeThreads / 32, std::max(1, (h.edges / std::max(1, h.levels) + 31) / 32));
+    const int slots = tab >= kEdgeSmem ? 0
+                                       : (int)std::min<size_t>({(size_t)cbk::kEdgeMaxSlots, (kEdgeSmem - tab) / per,
+                                                                (size_t)(cbk::kEdgeThreads / (32 * warps))});
+    if (slots >= 1 && h.max_row_degree <= 255) return ensure_edges(c, max_level_edges, slots, warps);
   }
   // the launch shape decides the message layout: a thread per row with messages in
   // global memory takes the transposed one
@@ -256,7 +320,7 @@ cb_status ensure_device(cb_ldpc* c) {
     const size_t per = (h.n + (size_t)(c->has_aux ? 2 : 1) * h.edges) * elem(c);
     c->group = (int)std::min<size_t>(cbk::kMaxGroup, kGroupSmem / per);
     if (c->group >= 2) {
-      c->kernel = cbk::sparse_group_kernel_ptr(c->precision == CB_F64 ? 0 : 1, c->rule, c->regs);
+      c->kernel = cbk::sparse_group_kernel_ptr(c->precision == CB_F64 ? 0 : 1, c->rule);
       c->smem = (c->group * per + 15) & ~(size_t)15;
       c->threads = std::min(512, (c->group * h.max_level_rows + 31) / 32 * 32);
     } else {
@@ -297,6 +361,25 @@ cb_status decode_impl(cb_ldpc* c, const T* llr, int64_t n, T* post, int32_t* ite
     a.work_counter = c->d_counter;
     LDPC_CUDA(c, cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned long long), s));
     LDPC_CUDA(c, cbk::launch_sparse(c->kernel, &a, (int)std::min<int64_t>(c->grid, n), c->threads, c->smem, s));
+    return CB_OK;
+  }
+  if (c->edge_slots) {
+    cbk::EdgeArgs<T> a;
+    a.code = c->edge;
+    a.max_iterations = c->max_iterations;
+    // few codewords are spread over the SMs first
+    a.slots = (int32_t)std::min<int64_t>(c->edge_slots, (n + c->grid - 1) / c->grid);
+    a.llr = llr;
+    a.n_frames = n;
+    a.post_out = post;
+    a.iters_out = iters;
+    a.work_counter = c->d_counter;
+    const size_t smem =
+        a.slots * cbk::sparse_edges_slot_bytes(c->edge.n, c->edge.edges, c->edge.max_level_edges, sizeof(T) == 8 ? 0 : 1) +
+        cbk::sparse_edges_table_bytes(c->edge.edges, c->edge.m, c->edge.levels);
+    LDPC_CUDA(c, cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned long long), s));
+    LDPC_CUDA(c, cbk::launch_sparse(c->kernel, &a, (int)std::min<int64_t>(c->grid, (n + a.slots - 1) / a.slots),
+                                    a.slots * c->edge.warps * 32, smem, s));
     return CB_OK;
   }
   cbk::SparseArgs<T> a;

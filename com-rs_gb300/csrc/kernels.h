@@ -219,8 +219,32 @@ void* sparse_kernel_ptr(int precision, int rule, bool layered, bool regs);
 // the layered kernel with several codewords per CTA (small codes: messages and
 // posteriors of the group in shared memory, one thread per row)
 constexpr int kMaxGroup = 8;
-void* sparse_group_kernel_ptr(int precision, int rule, bool regs);
+void* sparse_group_kernel_ptr(int precision, int rule);
 cudaError_t launch_sparse(void* kernel, const void* args, int grid, int threads, size_t smem, cudaStream_t stream);
+
+// ---- layered sum-product of small codes, an edge per thread (sparse_edges.cu).  The edges
+// in the order of the level schedule, row after row.
+constexpr int kEdgeThreads = 768;  // of a CTA at most
+constexpr int kEdgeMaxSlots = 15;  // codewords of a CTA at most: named barriers 1 to 15
+struct EdgeDev {
+  int32_t n, m, edges, levels, max_level_edges, warps;  // warps per codeword
+  const uint32_t* edge;  // edges: the variable (bits 0-15), the place in the row (16-23), its degree (24-31)
+  const int32_t* row;    // m + 1: the rows' first edges
+  const int32_t* level;  // levels + 1: the levels' first edges
+};
+template <typename T>
+struct EdgeArgs {
+  EdgeDev code;
+  int32_t max_iterations, slots;  // codewords per CTA
+  const T* llr;
+  int64_t n_frames;
+  T* post_out;
+  int32_t* iters_out;
+  unsigned long long* work_counter;
+};
+size_t sparse_edges_slot_bytes(int n, int edges, int max_level_edges, int precision);
+size_t sparse_edges_table_bytes(int edges, int m, int levels);
+void* sparse_edges_kernel_ptr(int precision);
 
 // ---- layered decoding of chained rows (sparse_chain.cu): blocks of consecutive rows
 // whose variables are distinct, but for the last variable of a row and the second to last

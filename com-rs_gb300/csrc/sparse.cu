@@ -454,7 +454,8 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) sparse_kernel(con
 // group's codewords are spread over the threads, one row each, so that the warps run full
 // even when a level has few rows (every warp instruction costs the same issue and pipe
 // time whatever its active lanes).  Each codeword stops on its own syndrome: its rows
-// are skipped from then on.  Results equal sparse_kernel's.
+// are skipped from then on.  Results equal sparse_kernel's.  (The sum-product rule comes
+// here only with rows of more than 255 edges: sparse_edges.cu takes the others.)
 template <typename T>
 __device__ __forceinline__ void group_syndrome(const SparseDev& c, const T* base, size_t per, int G,
                                                const int* check, volatile int* fail) {
@@ -470,7 +471,7 @@ __device__ __forceinline__ void group_syndrome(const SparseDev& c, const T* base
 
 // two CTAs of up to 512 threads fit an SM in f32 (at most 64 registers); one in f64, whose
 // rows need more (without the bound the compiler held the f64 min-sum rows to 40 and spilled)
-template <typename T, int RULE, bool REGS>
+template <typename T, int RULE>
 __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) sparse_group_kernel(const __grid_constant__ SparseArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SparseDev& c = a.code;
@@ -522,9 +523,8 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1) sparse_group_kern
           if (!s_run[g]) continue;
           T* post = base + g * per;
           T* msg = post + c.n;
-          if constexpr (REGS) check_row_spa_regs<T, kRegRowDegree>(c, c.level_rows[r0 + j], r0 + j, post, msg);
-          else check_row<T, RULE, true>(c, c.level_rows[r0 + j], r0 + j, post, msg, nullptr,
-                                        a.has_aux ? msg + c.slots : nullptr, alpha);
+          check_row<T, RULE, true>(c, c.level_rows[r0 + j], r0 + j, post, msg, nullptr,
+                                   a.has_aux ? msg + c.slots : nullptr, alpha);
         }
         __syncthreads();
       }
@@ -574,16 +574,14 @@ void* sparse_kernel_ptr(int precision, int rule, bool layered, bool regs) {
 }
 
 template <typename T>
-void* sparse_group_kernel_for(int rule, bool regs) {
-  if (rule == cbd::RULE_SUM_PRODUCT)
-    return regs ? (void*)sparse_group_kernel<T, cbd::RULE_SUM_PRODUCT, true>
-                : (void*)sparse_group_kernel<T, cbd::RULE_SUM_PRODUCT, false>;
-  if (rule == cbd::RULE_NMS) return (void*)sparse_group_kernel<T, cbd::RULE_NMS, false>;
-  return (void*)sparse_group_kernel<T, cbd::RULE_OMS, false>;
+void* sparse_group_kernel_for(int rule) {
+  if (rule == cbd::RULE_SUM_PRODUCT) return (void*)sparse_group_kernel<T, cbd::RULE_SUM_PRODUCT>;
+  if (rule == cbd::RULE_NMS) return (void*)sparse_group_kernel<T, cbd::RULE_NMS>;
+  return (void*)sparse_group_kernel<T, cbd::RULE_OMS>;
 }
 
-void* sparse_group_kernel_ptr(int precision, int rule, bool regs) {
-  return precision == 0 ? sparse_group_kernel_for<double>(rule, regs) : sparse_group_kernel_for<float>(rule, regs);
+void* sparse_group_kernel_ptr(int precision, int rule) {
+  return precision == 0 ? sparse_group_kernel_for<double>(rule) : sparse_group_kernel_for<float>(rule);
 }
 
 cudaError_t launch_sparse(void* kernel, const void* args, int grid, int threads, size_t smem, cudaStream_t s) {
