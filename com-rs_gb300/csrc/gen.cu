@@ -36,6 +36,7 @@
 #include "crmath.cuh"
 #include "decode_common.cuh"
 #include "kernels.h"
+#include "nr_encode.cuh"
 #include "qam_f64.cuh"
 
 namespace cbk {
@@ -177,57 +178,7 @@ __device__ __forceinline__ void gen_one(const cbd::DevCode& c, const GenFrame<T>
     }
   }
   __syncthreads();
-  // the 32-row window of a packed Z-bit column from row r0 with shift s (rows past Z read 0)
-  auto window = [&](const uint32_t* col, int r0, int shift) -> uint32_t {
-    int o = r0 + shift;
-    o -= (o >= z) ? z : 0;
-    uint32_t win = window32(col, o);
-    const int nrows = min(32, z - r0);
-    if (o + nrows > z) win |= window32(col, 0) << (z - o);
-    return nrows == 32 ? win : (win & ((1u << nrows) - 1u));
-  };
-  // core syndromes over the systematic columns
-  for (int task = tid; task < 4 * wz; task += NT) {
-    const int L = task / wz, g = task - L * wz;
-    uint32_t acc = 0;
-    for (int t = c.layer_start[L]; t < c.layer_start[L + 1]; t++) {
-      const uint32_t en = c.entry[t];
-      const int j = (int)(en >> 16);
-      if (j < c.cols_k) acc ^= window(cwp + j * ws, g * 32, (int)(en & 0xffffu));
-    }
-    synp[L * ws + g] = acc;
-    if (g == wz - 1) synp[L * ws + wz] = 0u;
-  }
-  __syncthreads();
-  // core parity: block-circulant inverse of the core
-  for (int task = tid; task < 4 * wz; task += NT) {
-    const int blk = task / wz, g = task - blk * wz;
-    uint32_t acc = 0;
-    for (int t = 0; t < c.n_core_terms; t++) {
-      const uint32_t ct = c.core_term[t];
-      if ((int)(ct >> 20) != blk) continue;
-      acc ^= window(synp + (int)((ct >> 16) & 15u) * ws, g * 32, (int)(ct & 0xffffu));
-    }
-    uint32_t* col = cwp + (c.cols_k + blk) * ws;
-    col[g] = acc;
-    if (g == wz - 1) col[wz] = 0u;
-  }
-  __syncthreads();
-  // extension parity: row L >= 4 closes on its own column cols_k + L (shift 0) and reads
-  // only systematic and core parity columns
-  for (int task = 4 * wz + tid; task < c.rows_n * wz; task += NT) {
-    const int L = task / wz, g = task - L * wz;
-    uint32_t acc = 0;
-    for (int t = c.layer_start[L]; t < c.layer_start[L + 1]; t++) {
-      const uint32_t en = c.entry[t];
-      const int j = (int)(en >> 16);
-      if (j != c.cols_k + L) acc ^= window(cwp + j * ws, g * 32, (int)(en & 0xffffu));
-    }
-    uint32_t* col = cwp + (c.cols_k + L) * ws;
-    col[g] = acc;
-    if (g == wz - 1) col[wz] = 0u;
-  }
-  __syncthreads();
+  encode_packed_columns(c, cwp, synp, tid, NT);
   // the parity bits back to bytes, for the labels
   for (int v = c.k + tid; v < c.n_full; v += NT) {
     const int j = v / z, b = v - j * z;

@@ -92,6 +92,15 @@ struct GenFrame {
   int32_t exact;       // demapper: 1 exact (log-sum-exp), 0 max-log
 };
 
+// ---- blocks of information bytes to sent bytes (encode.cu)
+struct NrEncodeArgs {
+  cbd::DevCode code;
+  const uint8_t* info;  // [n_frames][K']
+  uint8_t* out;         // [n_frames][E]
+  int64_t n_frames;
+};
+cudaError_t launch_nr_encode(const NrEncodeArgs& a, cudaStream_t stream);
+
 // ---- mixed batches (mix.cu, gen.cu): codewords of different codes in one launch
 // per (code, modulation) pair: the generator's tables
 struct GenConfig {
