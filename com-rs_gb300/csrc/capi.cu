@@ -834,8 +834,8 @@ struct cb_nms {
   float* d_g = nullptr;
   float* d_m = nullptr;
   float* d_v = nullptr;
-  float* d_X = nullptr;
-  size_t X_cap = 0;
+  unsigned char* d_tape = nullptr;
+  size_t tape_cap = 0;
   float* d_P = nullptr;
   size_t P_cap = 0;
   float* d_c2v = nullptr;
@@ -858,16 +858,19 @@ struct cb_nms {
 
 namespace {
 
-cb_status nms_buffers(cb_nms* h, int64_t n, bool train) {
+// what the device buffers of n frames are for
+enum NmsUse { kNmsEvaluate, kNmsForward, kNmsTrain };
+
+cb_status nms_buffers(cb_nms* h, int64_t n, NmsUse use) {
   cb_code* c = h->code;
-  const size_t edges = (size_t)c->dev.n_entries * c->dev.z;
-  CB_CUDA(c, grow(h->d_c2v, h->c2v_cap, (size_t)n * edges * 4));
   CB_CUDA(c, grow(h->d_llr, h->llr_cap, (size_t)n * c->host.e * 4));
   CB_CUDA(c, grow(h->d_post, h->post_cap, (size_t)n * c->host.n_full * 4));
   CB_CUDA(c, grow(h->d_info, h->info_cap, (size_t)n * ((c->host.k_info + 31) / 32) * 4));
   CB_CUDA(c, grow(h->d_res, h->res_cap, (size_t)n * sizeof(cbd::FrameResult)));
-  if (train) {
-    CB_CUDA(c, grow(h->d_X, h->X_cap, (size_t)n * h->T * edges * 4));
+  if (use != kNmsEvaluate)
+    CB_CUDA(c, grow(h->d_tape, h->tape_cap, (size_t)n * (use == kNmsTrain ? h->T : 1) * cbk::learned_tape_bytes(c->dev)));
+  if (use == kNmsTrain) {
+    CB_CUDA(c, grow(h->d_c2v, h->c2v_cap, (size_t)n * c->dev.n_entries * c->dev.z * 4));
     CB_CUDA(c, grow(h->d_P, h->P_cap, (size_t)n * h->T * c->host.n_full * 4));
     CB_CUDA(c, grow(h->d_cw, h->cw_cap, (size_t)n * ((c->host.n_full + 31) / 32) * 4));
     CB_CUDA(c, grow(h->d_ebn0, h->ebn0_cap, (size_t)n * 4));
@@ -992,11 +995,14 @@ cbk::LearnedArgs nms_args(cb_nms* h, int64_t n) {
   a.code = h->code->dev;
   a.T = h->T;
   a.shared = h->shared;
-  a.early_stop = 0;
   a.alpha = h->d_w;
   a.beta = h->d_w + h->nw;
   a.llr = h->d_llr;
   a.n_frames = n;
+  // one iteration's records, each replaced by the next (nms_fwd_bwd keeps all)
+  a.tape = h->d_tape;
+  a.tape_frame = cbk::learned_tape_bytes(h->code->dev);
+  a.tape_iter = 0;
   a.c2v = h->d_c2v;
   a.post_out = h->d_post;
   a.g_alpha = h->d_g;
@@ -1005,21 +1011,20 @@ cbk::LearnedArgs nms_args(cb_nms* h, int64_t n) {
   return a;
 }
 
-// forward (+ backward) of n frames already in d_llr / d_cw; loss into d_loss
-cb_status nms_fwd_bwd(cb_nms* h, int64_t n, bool backward, int multi, cudaStream_t s) {
+// forward and backward of n frames already in d_llr / d_cw; loss into d_loss
+cb_status nms_fwd_bwd(cb_nms* h, int64_t n, int multi, cudaStream_t s) {
   cb_code* c = h->code;
   cbk::LearnedArgs a = nms_args(h, n);
   a.cw_bits = h->d_cw;
-  a.X = backward ? h->d_X : nullptr;
+  a.tape_iter = cbk::learned_tape_bytes(c->dev);
+  a.tape_frame = (size_t)h->T * a.tape_iter;
   a.loss = h->d_loss;
   a.P = h->d_P;
   a.multi_loss = multi;
   CB_CUDA(c, cudaMemsetAsync(h->d_loss, 0, sizeof(float), s));
   CB_CUDA(c, cbk::launch_learned(a, true, s));
-  if (backward) {
-    CB_CUDA(c, cudaMemsetAsync(h->d_g, 0, sizeof(float) * 2 * h->nw, s));
-    CB_CUDA(c, cbk::launch_learned(a, false, s));
-  }
+  CB_CUDA(c, cudaMemsetAsync(h->d_g, 0, sizeof(float) * 2 * h->nw, s));
+  CB_CUDA(c, cbk::launch_learned(a, false, s));
   return CB_OK;
 }
 
@@ -1061,7 +1066,7 @@ cb_status cb_nms_create(cb_code* c, int32_t iterations, int32_t shared, cb_nms**
 void cb_nms_destroy(cb_nms* h) {
   if (!h) return;
   cudaSetDevice(h->code->device);
-  void* bufs[] = {h->d_w, h->d_g, h->d_m, h->d_v, h->d_X, h->d_P, h->d_c2v, h->d_post, h->d_llr, h->d_cw, h->d_info,
+  void* bufs[] = {h->d_w, h->d_g, h->d_m, h->d_v, h->d_tape, h->d_P, h->d_c2v, h->d_post, h->d_llr, h->d_cw, h->d_info,
                   h->d_ebn0, h->d_loss, h->d_res};
   for (void* p : bufs)
     if (p) cudaFree(p);
@@ -1107,7 +1112,7 @@ cb_status cb_nms_forward(cb_nms* h, const float* llr, int64_t n, float* post) {
   std::lock_guard<std::mutex> lock(c->mu);
   CB_CUDA(c, cudaSetDevice(c->device));
   if (n == 0) return CB_OK;
-  if (cb_status st = nms_buffers(h, n, false)) return st;
+  if (cb_status st = nms_buffers(h, n, kNmsForward)) return st;
   CB_CUDA(c, cudaMemcpyAsync(h->d_llr, llr, (size_t)n * c->host.e * 4, cudaMemcpyHostToDevice, c->stream));
   cbk::LearnedArgs a = nms_args(h, n);
   CB_CUDA(c, cbk::launch_learned(a, true, c->stream));
@@ -1129,7 +1134,7 @@ cb_status cb_nms_gradients(cb_nms* h, const float* llr, const uint8_t* cw, int64
   cb_code* c = h->code;
   std::lock_guard<std::mutex> lock(c->mu);
   CB_CUDA(c, cudaSetDevice(c->device));
-  if (cb_status st = nms_buffers(h, n, true)) return st;
+  if (cb_status st = nms_buffers(h, n, kNmsTrain)) return st;
   const int wpc = (c->host.n_full + 31) / 32;
   h->h_words.assign((size_t)n * wpc, 0u);
   for (int64_t f = 0; f < n; f++)
@@ -1137,7 +1142,7 @@ cb_status cb_nms_gradients(cb_nms* h, const float* llr, const uint8_t* cw, int64
       if (cw[(size_t)f * c->host.n_full + v] & 1) h->h_words[(size_t)f * wpc + v / 32] |= 1u << (v % 32);
   CB_CUDA(c, cudaMemcpyAsync(h->d_llr, llr, (size_t)n * c->host.e * 4, cudaMemcpyHostToDevice, c->stream));
   CB_CUDA(c, cudaMemcpyAsync(h->d_cw, h->h_words.data(), h->h_words.size() * 4, cudaMemcpyHostToDevice, c->stream));
-  if (cb_status st = nms_fwd_bwd(h, n, true, multi_loss, c->stream)) return st;
+  if (cb_status st = nms_fwd_bwd(h, n, multi_loss, c->stream)) return st;
   float l = 0.f;
   CB_CUDA(c, cudaMemcpyAsync(&l, h->d_loss, 4, cudaMemcpyDeviceToHost, c->stream));
   if (g_alpha) CB_CUDA(c, cudaMemcpyAsync(g_alpha, h->d_g, sizeof(float) * h->nw, cudaMemcpyDeviceToHost, c->stream));
@@ -1157,7 +1162,7 @@ cb_status cb_nms_train_step(cb_nms* h, int32_t m, uint64_t seed, uint64_t name_h
   CB_CUDA(c, cudaSetDevice(c->device));
   GenCache* g;
   if (cb_status st = gen_config(c, m, &g)) return st;
-  if (cb_status st = nms_buffers(h, batch, true)) return st;
+  if (cb_status st = nms_buffers(h, batch, kNmsTrain)) return st;
   // per-frame Eb/N0, uniform in [lo, hi], from a SplitMix64 sequence of (seed, step)
   std::vector<float> eb((size_t)batch);
   uint64_t st = seed ^ (0x9E3779B97F4A7C15ull * (uint64_t)(h->step + 1));
@@ -1168,7 +1173,7 @@ cb_status cb_nms_train_step(cb_nms* h, int32_t m, uint64_t seed, uint64_t name_h
   if (cb_status s2 = gen_device<float>(c, g, seed, name_hash, ~0ull, (uint64_t)h->step * batch, batch, lo, h->d_llr,
                                        h->d_info, c->stream, h->d_ebn0, h->d_cw))
     return s2;
-  if (cb_status s3 = nms_fwd_bwd(h, batch, true, multi_loss, c->stream)) return s3;
+  if (cb_status s3 = nms_fwd_bwd(h, batch, multi_loss, c->stream)) return s3;
   h->step++;
   h->h_w_valid = false;
   CB_CUDA(c, cbk::launch_adam(h->d_w, h->d_g, h->d_m, h->d_v, 2 * h->nw, (float)lr, h->step, c->stream));
@@ -1191,7 +1196,7 @@ cb_status cb_nms_decode(cb_nms* h, const float* llr, int64_t n, float* post, int
   const int64_t chunk = 16384;
   for (int64_t done = 0; done < n; done += chunk) {
     const int64_t cnt = std::min(chunk, n - done);
-    if (cb_status st = nms_buffers(h, cnt, false)) return st;
+    if (cb_status st = nms_buffers(h, cnt, kNmsEvaluate)) return st;
     CB_CUDA(c, grow(c->d_iters, c->iters_cap, (size_t)cnt * 4));
     CB_CUDA(c, cudaMemcpyAsync(h->d_llr, llr + (size_t)done * c->host.e, (size_t)cnt * c->host.e * 4,
                                cudaMemcpyHostToDevice, c->stream));
@@ -1237,7 +1242,7 @@ cb_status cb_nms_run_frames(cb_nms* h, int32_t m, uint64_t seed, uint64_t name_h
   const int64_t chunk = 16384;
   for (int64_t done = 0; done < n; done += chunk) {
     int64_t cnt = std::min(chunk, n - done);
-    if (cb_status st = nms_buffers(h, cnt, false)) return st;
+    if (cb_status st = nms_buffers(h, cnt, kNmsEvaluate)) return st;
     if (cb_status st = gen_device<float>(c, g, seed, name_hash, cond, first + done, cnt, ebn0_db, h->d_llr, h->d_info,
                                          c->stream))
       return st;

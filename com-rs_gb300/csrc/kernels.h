@@ -157,19 +157,22 @@ int mix_decode_grid(size_t smem, int device);
 cudaError_t launch_mix_decode(const MixDecodeArgs& a, int grid, size_t smem, cudaStream_t stream);
 size_t gen_smem_bytes(const cbd::DevCode& c, int m, int mbits, int n_pad);
 
-// Learned min-sum (nms_learned.cu): forward (training or evaluation) and backward.
+// Learned min-sum (nms_learned.cu): the training forward (also the posteriors of all T
+// iterations) and backward.
 struct LearnedArgs {
   cbd::DevCode code;
   int32_t T;           // unrolled iterations
   int32_t shared;      // 1: weights per base-graph edge, 0: per lifted edge
-  int32_t early_stop;  // 1: syndrome stop after each iteration (evaluation)
   const float* alpha;  // scales, then
   const float* beta;   // offsets
   const float* llr;    // [n_frames][E]
   int64_t n_frames;
   const uint32_t* cw_bits;  // [n_frames][ceil(n_full/32)] targets (training)
-  float* X;                 // [n_frames][T][edges] saved inputs (training)
-  float* c2v;               // [n_frames][edges] messages, then their gradients
+  // the row records, learned_tape_bytes per frame and iteration: iteration t of frame f at
+  // f tape_frame + t tape_iter (tape_iter 0: each iteration's replace the one's before)
+  unsigned char* tape;
+  size_t tape_frame, tape_iter;
+  float* c2v;               // [n_frames][edges] the messages' gradients (backward)
   float* post_out;          // [n_frames][n_full]
   float* loss;              // sum over frames of the mean bit loss (training)
   float* P;                 // [n_frames][T][n_full] posteriors after each iteration (multi-loss)
@@ -177,11 +180,8 @@ struct LearnedArgs {
   int32_t loss_bits;        // the loss covers codeword bits [0, loss_bits): n_full, or K' (the information bits)
   float* g_alpha;           // gradients of the mean loss (backward)
   float* g_beta;
-  const uint32_t* ref_bits;   // evaluation: sent info bits
-  cbd::FrameResult* results;  // evaluation records
-  int32_t* iters_out;
 };
-size_t learned_smem_bytes(const cbd::DevCode& code);
+inline size_t learned_tape_bytes(const cbd::DevCode& c) { return (((size_t)c.rows_n * c.z * 12) + 15) & ~(size_t)15; }
 cudaError_t launch_learned(const LearnedArgs& a, bool forward, cudaStream_t stream);
 cudaError_t launch_adam(float* w, const float* g, float* m, float* v, int64_t n, float lr, int step,
                         cudaStream_t stream);

@@ -21,6 +21,21 @@
 //   g_y = g_post[v] + g_c2v, g_a = g_y s [a > 0], dL/dalpha += g_a m, dL/dbeta -= g_a,
 //   g_m = g_a alpha flows to |x| of the argmin (or of the second argmin for the argmin),
 //   g_x = g_post[v] + sign(x) g_|x|, then g_post[v] = g_x and g_c2v = -g_x.
+//
+// The tape.  Everything the backward pass needs of a row is a function of its smallest and
+// second smallest |x|, their edges and the signs of x, so the forward pass saves these, 12
+// bytes a row and iteration (a plane of the two magnitudes, a plane of meta words), instead
+// of x itself, 4 bytes an edge (BG1: 27 bytes a row), and reads the previous iteration's
+// record where it kept the messages before: y follows from it and the previous iteration's
+// weights, the same bits.
+//
+// Bound: the latency of a frame's chain of rows (levels of one to three rows, a barrier
+// after each) at the residency that the posteriors allow, then issue.  Measured on GB300,
+// shared weights: 512 frames of BG1 Z = 384, 8 iterations, forward 3.57 -> 1.53 ms and
+// backward 6.52 -> 2.25 ms; 1024 frames of BG2 Z = 52, 10 iterations, 0.98 -> 0.48 and
+// 1.78 -> 0.79 ms (before: x on the tape, messages and weights read from global memory in
+// the rows, ten shuffles per edge for the weight gradients and their sums by shared-memory
+// atomics).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -31,10 +46,13 @@
 namespace cbk {
 namespace {
 
-__device__ __forceinline__ size_t weight_index(const LearnedArgs& a, int t, int entry, int r) {
-  return a.shared ? (size_t)t * a.code.n_entries + entry
-                  : ((size_t)t * a.code.n_entries + entry) * a.code.z + r;
-}
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kMaxDegree = 19;
+// the edges of a level at most (the dense core rows of base graph 1)
+constexpr int kMaxLevelEdges = 19;
+// meta word: bits 0-4 the first edge of the smallest |x|, bits 5-9 that of the second
+// smallest, bits 10.. the signs (x < 0)
+constexpr int kMetaSigns = 10;
 
 // weight of iteration t's output in the multi-loss: 1/T each (mode 1), or a linear ramp
 // 2 (t + 1) / (T (T + 1)) that leans on the last iterations (mode 2)
@@ -45,183 +63,219 @@ __device__ __forceinline__ float iter_loss_weight(int mode, int t, int T) {
 __device__ __forceinline__ float softplus_f(float x) { return x > 0.f ? x + log1pf(__expf(-x)) : log1pf(__expf(x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf(-x)); }
 
-// forward of one lifted row, degree D
-template <int D>
-__device__ __forceinline__ void learned_row_fwd(const LearnedArgs& a, float* post, float* c2v, float* X, int t,
-                                                int s0, int r, int z) {
-  int off[D];
-  float x[D];
-#pragma unroll
-  for (int e = 0; e < D; e++) {
-    const uint32_t en = a.code.entry[s0 + e];
-    unsigned cc = (unsigned)r + (en & 0xffffu);
-    unsigned cm = cc - (unsigned)z;
-    off[e] = (int)(en >> 16) * z + (int)min(cc, cm);
-    const size_t ed = (size_t)(s0 + e) * z + r;
-    float old = t > 0 ? c2v[ed] : 0.f;
-    x[e] = __fsub_rn(post[off[e]], old);
-    if (X) X[(size_t)t * a.code.n_entries * z + ed] = x[e];
+// the records of one frame and iteration: {m1, m2} per lifted row, then the meta words
+struct Tape {
+  float2* mag;
+  uint32_t* meta;
+  __device__ __forceinline__ Tape(unsigned char* base, int lifted)
+      : mag(reinterpret_cast<float2*>(base)), meta(reinterpret_cast<uint32_t*>(base + (size_t)lifted * 8)) {}
+};
+
+// the posteriors (or their gradients) at the start of a kernel's shared memory
+__host__ __device__ inline size_t learned_post_bytes(int n_full) { return ((size_t)n_full * 4 + 15) & ~(size_t)15; }
+
+// The (scale, offset) of entry i for lifted row r in one iteration: shared weights staged
+// in shared memory as pairs, or one per lifted edge in global memory.
+template <bool SHARED>
+struct RowWeights;
+template <>
+struct RowWeights<true> {
+  const float2* w;
+  __device__ __forceinline__ float2 at(int i, int, int) const { return w[i]; }
+};
+template <>
+struct RowWeights<false> {
+  const float *al, *be;
+  __device__ __forceinline__ float2 at(int i, int z, int r) const {
+    const size_t k = (size_t)i * z + r;
+    return make_float2(al[k], be[k]);
   }
-  uint32_t par = 0;
-  float m1 = INFINITY, m2 = INFINITY;
-  int i1 = 0;
-#pragma unroll
-  for (int e = 0; e < D; e++) {
-    par ^= (uint32_t)(x[e] < 0.f);
-    float av = fabsf(x[e]);
-    bool lt = av < m1;
-    m2 = lt ? m1 : fminf(m2, av);
-    m1 = lt ? av : m1;
-    i1 = lt ? e : i1;
-  }
-#pragma unroll
-  for (int e = 0; e < D; e++) {
-    const size_t w = weight_index(a, t, s0 + e, r);
-    float m = e == i1 ? m2 : m1;
-    float am = __fmaf_rn(a.alpha[w], m, -a.beta[w]);
-    float mag = am > 0.f ? am : 0.f;
-    bool neg = (par ^ (uint32_t)(x[e] < 0.f)) & 1u;
-    float y = neg ? -mag : mag;
-    c2v[(size_t)(s0 + e) * z + r] = y;
-    post[off[e]] = __fadd_rn(x[e], y);
-  }
+};
+
+// the message of edge e from its row's record
+__device__ __forceinline__ float learned_message(float2 w, float m, uint32_t neg) {
+  const float am = __fmaf_rn(w.x, m, -w.y);
+  const float mag = am > 0.f ? am : 0.f;
+  return neg ? -mag : mag;
 }
 
-template <int D>
-__device__ __forceinline__ void learned_row_bwd(const LearnedArgs& a, float* gp, float* gc, const float* X, int t,
-                                                int s0, int r, int z, float* sga, float* sgb) {
+// forward of one lifted row, degree D, entries s0 ..; (o1, o2, om) the previous
+// iteration's record
+template <int D, bool SHARED>
+__device__ __forceinline__ void learned_row_fwd(const LearnedArgs& a, float* post, int s0, int r, int z, bool first,
+                                                const RowWeights<SHARED>& wp, const RowWeights<SHARED>& wc, float2 o,
+                                                uint32_t om, float2& n, uint32_t& nm) {
+  const EdgeAddrTable addr{a.code.eaddr + s0, r, 4 * r, 4 * z};
   int off[D];
   float x[D];
-#pragma unroll
-  for (int e = 0; e < D; e++) {
-    const uint32_t en = a.code.entry[s0 + e];
-    unsigned cc = (unsigned)r + (en & 0xffffu);
-    unsigned cm = cc - (unsigned)z;
-    off[e] = (int)(en >> 16) * z + (int)min(cc, cm);
-    x[e] = X[(size_t)t * a.code.n_entries * z + (size_t)(s0 + e) * z + r];
-  }
-  uint32_t par = 0;
+  const int oi1 = (int)(om & 31u);
+  const uint32_t os = om >> kMetaSigns, op = __popc(os) & 1u;
+  uint32_t sg = 0;
   float m1 = INFINITY, m2 = INFINITY;
   int i1 = 0, i2 = 0;
 #pragma unroll
   for (int e = 0; e < D; e++) {
-    par ^= (uint32_t)(x[e] < 0.f);
-    float av = fabsf(x[e]);
-    if (av < m1) {
-      m2 = m1;
-      i2 = i1;
-      m1 = av;
-      i1 = e;
-    } else if (av < m2) {
-      m2 = av;
-      i2 = e;
-    }
-  }
-  float g1 = 0.f, g2 = 0.f;  // gradients of |x_i1| and |x_i2|
-#pragma unroll
-  for (int e = 0; e < D; e++) {
-    const size_t w = weight_index(a, t, s0 + e, r);
-    const size_t ed = (size_t)(s0 + e) * z + r;
-    float m = e == i1 ? m2 : m1;
-    float al = a.alpha[w];
-    float am = __fmaf_rn(al, m, -a.beta[w]);
-    bool neg = (par ^ (uint32_t)(x[e] < 0.f)) & 1u;
-    float gy = gp[off[e]] + gc[ed];
-    float ga = am > 0.f ? (neg ? -gy : gy) : 0.f;
-    if (a.shared) {
-      sga[e] = ga * m;
-      sgb[e] = -ga;
-    } else {
-      atomicAdd(&a.g_alpha[w], ga * m);
-      atomicAdd(&a.g_beta[w], -ga);
-    }
-    float gm = ga * al;
-    if (e == i1) g2 += gm;
-    else g1 += gm;
+    off[e] = addr(e);
+    float old = 0.f;
+    if (!first) old = learned_message(wp.at(s0 + e, z, r), e == oi1 ? o.y : o.x, op ^ ((os >> e) & 1u));
+    x[e] = __fsub_rn(ld_post(post, off[e]), old);
   }
 #pragma unroll
   for (int e = 0; e < D; e++) {
-    float gabs = (e == i1 ? g1 : 0.f) + (e == i2 && i2 != i1 ? g2 : 0.f);
-    float gx = gp[off[e]] + (x[e] < 0.f ? -gabs : gabs);
-    gp[off[e]] = gx;
-    gc[(size_t)(s0 + e) * z + r] = -gx;
+    sg |= (uint32_t)(x[e] < 0.f) << e;
+    const float av = fabsf(x[e]);
+    const bool lt1 = av < m1, lt2 = av < m2;
+    m2 = lt1 ? m1 : lt2 ? av : m2;
+    i2 = lt1 ? i1 : lt2 ? e : i2;
+    m1 = lt1 ? av : m1;
+    i1 = lt1 ? e : i1;
   }
-}
-
-template <bool FWD>
-__device__ __forceinline__ void learned_row(int d, const LearnedArgs& a, float* p, float* c, float* X, int t, int s0,
-                                            int r, int z, float* sga, float* sgb) {
-#define CB_LROW(DD)                                                       \
-  case DD:                                                                \
-    if (FWD) learned_row_fwd<DD>(a, p, c, X, t, s0, r, z);                \
-    else learned_row_bwd<DD>(a, p, c, X, t, s0, r, z, sga, sgb);          \
-    break;
-  switch (d) {
-    CB_LROW(3)
-    CB_LROW(4)
-    CB_LROW(5)
-    CB_LROW(6)
-    CB_LROW(7)
-    CB_LROW(8)
-    CB_LROW(9)
-    CB_LROW(10)
-    default:
-      if (FWD) learned_row_fwd<19>(a, p, c, X, t, s0, r, z);
-      else learned_row_bwd<19>(a, p, c, X, t, s0, r, z, sga, sgb);
-  }
-#undef CB_LROW
-}
-
-// Shared weights: the row gradients of a layer summed over its Z threads (warp shuffles,
-// one shared-memory add per warp), then one global add per entry.
-__device__ __forceinline__ void reduce_shared_grads(const LearnedArgs& a, int t, int s0, int d, const float* sga,
-                                                    const float* sgb, float* red, int tid, bool active) {
-  const int lane = tid & 31;
-  for (int e = 0; e < 19; e++) {
-    if (e >= d) break;
-    float va = active ? sga[e] : 0.f, vb = active ? sgb[e] : 0.f;
+  const uint32_t par = __popc(sg) & 1u;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      va += __shfl_xor_sync(0xffffffffu, va, o);
-      vb += __shfl_xor_sync(0xffffffffu, vb, o);
+  for (int e = 0; e < D; e++) {
+    const float y = learned_message(wc.at(s0 + e, z, r), e == i1 ? m2 : m1, par ^ ((sg >> e) & 1u));
+    st_post(post, off[e], __fadd_rn(x[e], y));
+  }
+  n = make_float2(m1, m2);
+  nm = (uint32_t)i1 | (uint32_t)i2 << 5 | sg << kMetaSigns;
+}
+
+// The sums of N values over the warp's lanes in about N + 5 shuffles: each step halves
+// the values a lane holds, the lanes of one half keeping the first half's sums and the others
+// the second's.  Lane l is left with v[j] = the sum of value index(j), j < (N + 31) / 32.
+template <int N, int O>
+struct WarpSums {
+  static constexpr int H = (N + 1) / 2;
+  using Next = WarpSums<H, O / 2>;
+  static constexpr int left = Next::left;
+  static __device__ __forceinline__ void sum(float* v, int lane) {
+    const bool up = (lane & O) != 0;
+#pragma unroll
+    for (int i = 0; i < H; i++) {
+      if (i + H < N) {
+        const float send = up ? v[i] : v[i + H], keep = up ? v[i + H] : v[i];
+        v[i] = keep + __shfl_xor_sync(kFull, send, O);
+      } else {
+        v[i] += __shfl_xor_sync(kFull, v[i], O);
+      }
     }
-    if (lane == 0) {
-      atomicAdd(&red[2 * e], va);
-      atomicAdd(&red[2 * e + 1], vb);
+    Next::sum(v, lane);
+  }
+  // the value that slot j of this lane sums, -1 for a copy of another lane's
+  static __device__ __forceinline__ int index(int j, int lane) {
+    const int i = Next::index(j, lane);
+    if (i < 0) return -1;
+    if ((lane & O) == 0) return i;
+    return i + H < N ? i + H : -1;
+  }
+};
+template <int N>
+struct WarpSums<N, 0> {
+  static constexpr int left = N;
+  static __device__ __forceinline__ void sum(float*, int) {}
+  static __device__ __forceinline__ int index(int j, int) { return j; }
+};
+
+// Backward of one lifted row from its record.  With shared weights `red` receives the
+// warp's sums of the gradients: D scales, then D offsets (every lane of the warp takes part;
+// the lanes without a row with zeros).
+template <int D, bool SHARED>
+__device__ __forceinline__ void learned_row_bwd(const LearnedArgs& a, float* gp, float* gc, float2 n, uint32_t nm,
+                                                int t, int s0, int r, int z, bool active, bool last,
+                                                const RowWeights<SHARED>& w, float* red, int lane) {
+  float v[2 * D];  // the gradients of the scales, then of the offsets
+#pragma unroll
+  for (int i = 0; i < 2 * D; i++) v[i] = 0.f;
+  if (active) {
+    const EdgeAddrTable addr{a.code.eaddr + s0, r, 4 * r, 4 * z};
+    int off[D];
+    float gy[D];
+    const int i1 = (int)(nm & 31u), i2 = (int)((nm >> 5) & 31u);
+    const uint32_t sg = nm >> kMetaSigns, par = __popc(sg) & 1u;
+#pragma unroll
+    for (int e = 0; e < D; e++) gy[e] = last ? 0.f : gc[(size_t)(s0 + e) * z + r];
+    float g1 = 0.f, g2 = 0.f;  // gradients of |x_i1| and |x_i2|
+#pragma unroll
+    for (int e = 0; e < D; e++) {
+      off[e] = addr(e);
+      gy[e] = ld_post(gp, off[e]) + gy[e];
+      const float2 ab = w.at(s0 + e, z, r);
+      const float m = e == i1 ? n.y : n.x;
+      const float am = __fmaf_rn(ab.x, m, -ab.y);
+      const float g = (par ^ ((sg >> e) & 1u)) ? -gy[e] : gy[e];
+      const float ga = am > 0.f ? g : 0.f;
+      if constexpr (SHARED) {
+        v[e] = ga * m;
+        v[D + e] = -ga;
+      } else {
+        const size_t k = ((size_t)t * a.code.n_entries + s0 + e) * z + r;
+        atomicAdd(&a.g_alpha[k], ga * m);
+        atomicAdd(&a.g_beta[k], -ga);
+      }
+      const float gm = ga * ab.x;
+      if (e == i1) g2 += gm;
+      else g1 += gm;
+    }
+#pragma unroll
+    for (int e = 0; e < D; e++) {
+      const float gabs = (e == i1 ? g1 : 0.f) + (e == i2 && i2 != i1 ? g2 : 0.f);
+      const float gx = ld_post(gp, off[e]) + (((sg >> e) & 1u) ? -gabs : gabs);
+      st_post(gp, off[e], gx);
+      if (t > 0) gc[(size_t)(s0 + e) * z + r] = -gx;
     }
   }
-  __syncthreads();
-  if (tid < d) {
-    const size_t w = (size_t)t * a.code.n_entries + s0 + tid;
-    atomicAdd(&a.g_alpha[w], red[2 * tid]);
-    atomicAdd(&a.g_beta[w], red[2 * tid + 1]);
-    red[2 * tid] = 0.f;
-    red[2 * tid + 1] = 0.f;
+  if constexpr (SHARED) {
+    using S = WarpSums<2 * D, 16>;
+    S::sum(v, lane);
+#pragma unroll
+    for (int j = 0; j < S::left; j++) {
+      const int i = S::index(j, lane);
+      if (i >= 0) red[i] = v[j];
+    }
   }
 }
 
-__global__ void __launch_bounds__(384) learned_forward_kernel(const __grid_constant__ LearnedArgs a) {
+#define CB_LEARNED_DEGREES(ROW) \
+  switch (d) {                  \
+    case 3: ROW(3) break;       \
+    case 4: ROW(4) break;       \
+    case 5: ROW(5) break;       \
+    case 6: ROW(6) break;       \
+    case 7: ROW(7) break;       \
+    case 8: ROW(8) break;       \
+    case 9: ROW(9) break;       \
+    case 10: ROW(10) break;     \
+    default: ROW(19) break;     \
+  }
+
+// the weights of iteration t: staged in `buf` (shared; visible after the caller's next
+// barrier) or in global memory
+template <bool SHARED>
+__device__ __forceinline__ RowWeights<SHARED> iteration_weights(const LearnedArgs& a, float2* buf, int t) {
+  const int ne = a.code.n_entries;
+  if constexpr (SHARED) {
+    for (int i = threadIdx.x; i < ne; i += blockDim.x)
+      buf[i] = make_float2(a.alpha[(size_t)t * ne + i], a.beta[(size_t)t * ne + i]);
+    return {buf};
+  } else {
+    const size_t per = (size_t)ne * a.code.z;
+    return {a.alpha + t * per, a.beta + t * per};
+  }
+}
+
+template <bool SHARED>
+__global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_constant__ LearnedArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const cbd::DevCode& c = a.code;
   const int z = c.z, nt = blockDim.x, tid = threadIdx.x;
-  const int ncol = c.n_full / z, ws = (z + 31) / 32 + 1;
+  const int ne = c.n_entries, lifted = c.rows_n * z;
   float* post = reinterpret_cast<float*>(smem);
-  uint32_t* hd = reinterpret_cast<uint32_t*>(post + c.n_full);
-  uint32_t* s_ent = hd + ncol * ws;
-  uint16_t* s_lstart = reinterpret_cast<uint16_t*>(s_ent + c.n_entries);
+  float2* wbuf = reinterpret_cast<float2*>(smem + learned_post_bytes(c.n_full));  // two iterations' (shared)
   __shared__ float s_loss;
-  __shared__ unsigned int s_err;
   const long long f = blockIdx.x;
   if (f >= a.n_frames) return;
-  for (int i = tid; i < c.n_entries; i += nt) s_ent[i] = c.entry[i];
-  for (int i = tid; i <= c.rows_n; i += nt) s_lstart[i] = c.layer_start[i];
-  if (tid == 0) {
-    s_loss = 0.f;
-    s_err = 0;
-  }
-  const size_t edges = (size_t)c.n_entries * z;
-  float* c2v = a.c2v + (size_t)f * edges;
-  float* X = a.X ? a.X + (size_t)f * a.T * edges : nullptr;
+  if (tid == 0) s_loss = 0.f;
+  unsigned char* tape = a.tape + (size_t)f * a.tape_frame;
   const float* llr = a.llr + (size_t)f * c.e;
   for (int v = tid; v < c.n_full; v += nt) post[v] = 0.f;
   __syncthreads();
@@ -241,32 +295,57 @@ __global__ void __launch_bounds__(384) learned_forward_kernel(const __grid_const
   __syncthreads();
   for (int v = c.k_info + tid; v < c.k; v += nt) post[v] = cbd::kKnownBitLlr;
   __syncthreads();
-  int it = 0;
-  const bool stop = a.early_stop != 0;
   const bool multi = a.multi_loss && a.P && a.cw_bits && a.loss;
+  const bool active = tid < z;
   float lsum = 0.f;  // this thread's share of the loss
-  if (!stop || some_check_fails(post, hd, s_ent, s_lstart, c.rows_n, ncol, z, tid, nt)) {
-    it = a.T;
-    for (int t = 0; t < a.T; t++) {
-      for (int L = 0; L < c.rows_n; L++) {
-        if (tid < z) {
-          const int s0 = s_lstart[L];
-          learned_row<true>(s_lstart[L + 1] - s0, a, post, c2v, X, t, s0, tid, z, nullptr, nullptr);
-        }
-        __syncthreads();
+  RowWeights<SHARED> wp = iteration_weights<SHARED>(a, wbuf, 0), wc = wp;
+  for (int t = 0; t < a.T; t++) {
+    if (t > 0) {
+      wp = wc;
+      wc = iteration_weights<SHARED>(a, wbuf + (t & 1) * ne, t);
+    }
+    __syncthreads();
+    const Tape old(tape + (t > 0 ? (size_t)(t - 1) * a.tape_iter : 0), lifted);
+    const Tape cur(tape + (size_t)t * a.tape_iter, lifted);
+    // the next row's old record is loaded a row ahead
+    float2 o = make_float2(0.f, 0.f);
+    uint32_t om = 0;
+    if (active && t > 0) {
+      const int i = c.layer_order[0] * z + tid;
+      o = old.mag[i];
+      om = old.meta[i];
+    }
+    for (int q = 0; q < c.rows_n; q++) {
+      const int L = c.layer_order[q];
+      float2 on = o;
+      uint32_t omn = om;
+      if (active && t > 0 && q + 1 < c.rows_n) {
+        const int i = c.layer_order[q + 1] * z + tid;
+        on = old.mag[i];
+        omn = old.meta[i];
       }
-      if (multi) {
-        const int wpc = (c.n_full + 31) >> 5;
-        float* Pt = a.P + ((size_t)f * a.T + t) * c.n_full;
-        for (int v = tid; v < a.loss_bits; v += nt) {
-          Pt[v] = post[v];
-          int bit = (a.cw_bits[(size_t)f * wpc + (v >> 5)] >> (v & 31)) & 1;
-          lsum += softplus_f(bit ? post[v] : -post[v]) * iter_loss_weight(a.multi_loss, t, a.T);
-        }
+      if (active) {
+        const int s0 = c.layer_start[L], d = c.layer_start[L + 1] - s0;
+        float2 n;
+        uint32_t nm;
+#define CB_ROW(DD) learned_row_fwd<DD, SHARED>(a, post, s0, tid, z, t == 0, wp, wc, o, om, n, nm);
+        CB_LEARNED_DEGREES(CB_ROW)
+#undef CB_ROW
+        cur.mag[L * z + tid] = n;
+        cur.meta[L * z + tid] = nm;
       }
-      if (stop && !some_check_fails(post, hd, s_ent, s_lstart, c.rows_n, ncol, z, tid, nt)) {
-        it = t + 1;
-        break;
+      o = on;
+      om = omn;
+      if (c.level_end[q]) __syncthreads();
+    }
+    if (multi) {
+      const int wpc = (c.n_full + 31) >> 5;
+      const float wt = iter_loss_weight(a.multi_loss, t, a.T);
+      float* Pt = a.P + ((size_t)f * a.T + t) * c.n_full;
+      for (int v = tid; v < a.loss_bits; v += nt) {
+        Pt[v] = post[v];
+        int bit = (a.cw_bits[(size_t)f * wpc + (v >> 5)] >> (v & 31)) & 1;
+        lsum += softplus_f(bit ? post[v] : -post[v]) * wt;
       }
     }
   }
@@ -281,60 +360,37 @@ __global__ void __launch_bounds__(384) learned_forward_kernel(const __grid_const
         lsum += softplus_f(bit ? post[v] : -post[v]);
       }
     }
-    atomicAdd(&s_loss, lsum);
-  }
-  const int wpf = (c.k_info + 31) >> 5, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  unsigned int be = 0;
-  // the sent words, one per thread, loaded before the ballots so that their latency
-  // overlaps them; the decisions are staged in hd (free after the syndrome tests)
-  const uint32_t* ref = a.ref_bits ? a.ref_bits + (size_t)f * wpf : nullptr;
-  const uint32_t ref_w = (ref && tid < wpf) ? ref[tid] : 0u;
-  if (ref) {
-    for (int b0 = warp * 32; b0 < c.k_info; b0 += nw * 32) {
-      int v = b0 + lane;
-      uint32_t word = __ballot_sync(0xffffffffu, v < c.k_info && post[v] < 0.f);
-      if (lane == 0) hd[b0 >> 5] = word;
-    }
+    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(kFull, lsum, o);
+    if ((tid & 31) == 0) atomicAdd(&s_loss, lsum);
     __syncthreads();
-    if (tid < wpf) be = __popc(hd[tid] ^ ref_w);
-    for (int w = tid + nt; w < wpf; w += nt) be += __popc(hd[w] ^ ref[w]);
-  }
-  if (be) atomicAdd(&s_err, be);
-  __syncthreads();
-  if (tid == 0) {
-    if (a.loss && a.cw_bits) atomicAdd(a.loss, s_loss / (float)a.loss_bits);
-    if (a.iters_out) a.iters_out[f] = it;
-    if (a.results) {
-      cbd::FrameResult r;
-      r.bit_errors = s_err;
-      r.frame_error = s_err > 0;
-      r.iterations = (uint8_t)it;
-      r.reserved = 0;
-      a.results[f] = r;
-    }
+    if (tid == 0) atomicAdd(a.loss, s_loss / (float)a.loss_bits);
   }
 }
 
-__global__ void __launch_bounds__(384) learned_backward_kernel(const __grid_constant__ LearnedArgs a) {
+template <bool SHARED>
+__global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_constant__ LearnedArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const cbd::DevCode& c = a.code;
-  const int z = c.z, nt = blockDim.x, tid = threadIdx.x;
+  const int z = c.z, nt = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  const int lifted = c.rows_n * z;
   float* gp = reinterpret_cast<float*>(smem);
-  float* red = gp + c.n_full;  // 2 x 19 floats
+  float2* wbuf = reinterpret_cast<float2*>(smem + learned_post_bytes(c.n_full));
+  // the warps' sums of a level's weight gradients, in two buffers by turns (shared weights)
+  float* red = reinterpret_cast<float*>(wbuf + c.n_entries);
+  constexpr int RW = 2 * kMaxLevelEdges;
   const long long f = blockIdx.x;
   if (f >= a.n_frames) return;
   const size_t edges = (size_t)c.n_entries * z;
-  float* gc = a.c2v + (size_t)f * edges;  // the message gradients reuse the message buffer
-  const float* X = a.X + (size_t)f * a.T * edges;
+  float* gc = a.c2v + (size_t)f * edges;  // the message gradients
   const int wpc = (c.n_full + 31) >> 5;
   const bool multi = a.multi_loss && a.P;
+  const bool active = tid < z;
   const float scale = 1.f / ((float)a.loss_bits * (float)a.n_frames);
   for (int v = tid; v < c.n_full; v += nt) gp[v] = 0.f;
-  for (size_t i = tid; i < edges; i += nt) gc[i] = 0.f;
-  if (tid < 38) red[tid] = 0.f;
   __syncthreads();
-  float sga[19], sgb[19];
+  int buf = 0;
   for (int t = a.T - 1; t >= 0; t--) {
+    const RowWeights<SHARED> w = iteration_weights<SHARED>(a, wbuf, t);
     // the loss of iteration t's output (every iteration, or the last one)
     if (multi || t == a.T - 1) {
       const float* p = multi ? a.P + ((size_t)f * a.T + t) * c.n_full : a.post_out + (size_t)f * c.n_full;
@@ -344,13 +400,57 @@ __global__ void __launch_bounds__(384) learned_backward_kernel(const __grid_cons
         float sgn = bit ? -1.f : 1.f;
         gp[v] += -sgn * sigmoid_f(-sgn * p[v]) * sc;
       }
-      __syncthreads();
     }
-    for (int L = c.rows_n - 1; L >= 0; L--) {
-      const int s0 = c.layer_start[L], d = c.layer_start[L + 1] - s0;
-      if (tid < z) learned_row<false>(d, a, gp, gc, const_cast<float*>(X), t, s0, tid, z, sga, sgb);
-      if (a.shared) reduce_shared_grads(a, t, s0, d, sga, sgb, red, tid, tid < z);
+    __syncthreads();
+    const Tape cur(a.tape + (size_t)f * a.tape_frame + (size_t)t * a.tape_iter, lifted);
+    // the next row's record is loaded a row ahead
+    float2 n = make_float2(0.f, 0.f);
+    uint32_t nm = 0;
+    if (active) {
+      const int i = c.layer_order[c.rows_n - 1] * z + tid;
+      n = cur.mag[i];
+      nm = cur.meta[i];
+    }
+    for (int q = c.rows_n - 1; q >= 0;) {
+      // the rows of a level, then a barrier, then the level's sums into the gradients
+      int at = 0, qe = q;
+      do {
+        const int L = c.layer_order[qe];
+        const int s0 = c.layer_start[L], d = c.layer_start[L + 1] - s0;
+        float2 nn = n;
+        uint32_t nmn = nm;
+        if (active && qe > 0) {
+          const int i = c.layer_order[qe - 1] * z + tid;
+          nn = cur.mag[i];
+          nmn = cur.meta[i];
+        }
+        float* rd = red + ((size_t)buf * nw + warp) * RW + 2 * at;
+#define CB_ROW(DD) \
+  learned_row_bwd<DD, SHARED>(a, gp, gc, n, nm, t, s0, tid, z, active, t == a.T - 1, w, rd, lane);
+        CB_LEARNED_DEGREES(CB_ROW)
+#undef CB_ROW
+        n = nn;
+        nm = nmn;
+        at += d;
+        qe--;
+      } while (qe >= 0 && !c.level_end[qe]);
       __syncthreads();
+      if constexpr (SHARED) {
+        for (int base = 0; q > qe; q--) {
+          const int L = c.layer_order[q];
+          const int s0 = c.layer_start[L], d = c.layer_start[L + 1] - s0;
+          for (int i = tid; i < 2 * d; i += nt) {
+            const float* rd = red + (size_t)buf * nw * RW + 2 * base + i;
+            float s = 0.f;
+            for (int k = 0; k < nw; k++) s += rd[k * RW];
+            const size_t wi = (size_t)t * c.n_entries + s0 + (i < d ? i : i - d);
+            atomicAdd(i < d ? &a.g_alpha[wi] : &a.g_beta[wi], s);
+          }
+          base += d;
+        }
+        buf ^= 1;
+      }
+      q = qe;
     }
   }
 }
@@ -370,17 +470,14 @@ __global__ void adam_kernel(float* w, const float* g, float* m, float* v, int64_
 
 }  // namespace
 
-size_t learned_smem_bytes(const cbd::DevCode& c) {
-  const int ws = (c.z + 31) / 32 + 1;
-  size_t b = (size_t)c.n_full * 4 + (size_t)(c.n_full / c.z) * ws * 4 + (size_t)c.n_entries * 4 +
-             (size_t)(c.rows_n + 1) * 2 + 16;
-  return (b + 15) & ~(size_t)15;
-}
-
 cudaError_t launch_learned(const LearnedArgs& a, bool forward, cudaStream_t s) {
   const int threads = ((a.code.z + 31) / 32) * 32;
-  void* k = forward ? (void*)learned_forward_kernel : (void*)learned_backward_kernel;
-  size_t smem = forward ? learned_smem_bytes(a.code) : (size_t)a.code.n_full * 4 + 2 * 19 * 4 + 16;
+  void* k = forward ? (a.shared ? (void*)learned_forward_kernel<true> : (void*)learned_forward_kernel<false>)
+                    : (a.shared ? (void*)learned_backward_kernel<true> : (void*)learned_backward_kernel<false>);
+  size_t smem = learned_post_bytes(a.code.n_full);
+  if (a.shared)
+    smem += forward ? 2 * sizeof(float2) * a.code.n_entries
+                    : sizeof(float2) * a.code.n_entries + 2 * (size_t)(threads / 32) * 2 * kMaxLevelEdges * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void* args[] = {(void*)&a};
