@@ -853,7 +853,8 @@ struct cb_nms {
   float* d_loss = nullptr;
   cbd::FrameResult* d_res = nullptr;
   size_t res_cap = 0;
-  std::vector<uint32_t> h_words;
+  uint8_t* d_bytes = nullptr;  // codewords as the caller gives them
+  size_t bytes_cap = 0;
 };
 
 namespace {
@@ -1067,7 +1068,7 @@ void cb_nms_destroy(cb_nms* h) {
   if (!h) return;
   cudaSetDevice(h->code->device);
   void* bufs[] = {h->d_w, h->d_g, h->d_m, h->d_v, h->d_tape, h->d_P, h->d_c2v, h->d_post, h->d_llr, h->d_cw, h->d_info,
-                  h->d_ebn0, h->d_loss, h->d_res};
+                  h->d_ebn0, h->d_loss, h->d_res, h->d_bytes};
   for (void* p : bufs)
     if (p) cudaFree(p);
   delete h;
@@ -1135,13 +1136,10 @@ cb_status cb_nms_gradients(cb_nms* h, const float* llr, const uint8_t* cw, int64
   std::lock_guard<std::mutex> lock(c->mu);
   CB_CUDA(c, cudaSetDevice(c->device));
   if (cb_status st = nms_buffers(h, n, kNmsTrain)) return st;
-  const int wpc = (c->host.n_full + 31) / 32;
-  h->h_words.assign((size_t)n * wpc, 0u);
-  for (int64_t f = 0; f < n; f++)
-    for (int v = 0; v < c->host.n_full; v++)
-      if (cw[(size_t)f * c->host.n_full + v] & 1) h->h_words[(size_t)f * wpc + v / 32] |= 1u << (v % 32);
+  CB_CUDA(c, grow(h->d_bytes, h->bytes_cap, (size_t)n * c->host.n_full));
   CB_CUDA(c, cudaMemcpyAsync(h->d_llr, llr, (size_t)n * c->host.e * 4, cudaMemcpyHostToDevice, c->stream));
-  CB_CUDA(c, cudaMemcpyAsync(h->d_cw, h->h_words.data(), h->h_words.size() * 4, cudaMemcpyHostToDevice, c->stream));
+  CB_CUDA(c, cudaMemcpyAsync(h->d_bytes, cw, (size_t)n * c->host.n_full, cudaMemcpyHostToDevice, c->stream));
+  CB_CUDA(c, cbk::launch_pack_codewords(h->d_bytes, h->d_cw, n, c->host.n_full, c->stream));
   if (cb_status st = nms_fwd_bwd(h, n, multi_loss, c->stream)) return st;
   float l = 0.f;
   CB_CUDA(c, cudaMemcpyAsync(&l, h->d_loss, 4, cudaMemcpyDeviceToHost, c->stream));

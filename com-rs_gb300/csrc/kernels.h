@@ -183,6 +183,8 @@ struct LearnedArgs {
 };
 inline size_t learned_tape_bytes(const cbd::DevCode& c) { return (((size_t)c.rows_n * c.z * 12) + 15) & ~(size_t)15; }
 cudaError_t launch_learned(const LearnedArgs& a, bool forward, cudaStream_t stream);
+// codeword bytes [n_frames][n_bits] to packed words [n_frames][ceil(n_bits / 32)], LSB first
+cudaError_t launch_pack_codewords(const uint8_t* bytes, uint32_t* words, int64_t n_frames, int n_bits, cudaStream_t s);
 cudaError_t launch_adam(float* w, const float* g, float* m, float* v, int64_t n, float lr, int step,
                         cudaStream_t stream);
 template <typename T>
