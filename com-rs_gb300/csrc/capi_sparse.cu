@@ -175,12 +175,13 @@ cb_status ensure_chain(cb_ldpc* c, const cbh::ChainBlocks& blocks) {
 
 // The edge-parallel sum-product decoder (sparse_edges.cu): `slots` codewords per CTA, one
 // CTA per SM.
-cb_status ensure_edges(cb_ldpc* c, int max_level_edges, int slots, int warps) {
+cb_status ensure_edges(cb_ldpc* c, const cbh::LevelSchedule& sched, int max_level_edges, int slots, int warps) {
   const cbh::SparseCode& h = c->host;
+  const int levels = (int)sched.level_start.size() - 1;
   std::vector<int32_t> tab(h.edges), row(1, 0), level(1, 0);
-  for (int l = 0, e = 0; l < h.levels; l++) {
-    for (int i = h.level_start[l]; i < h.level_start[l + 1]; i++) {
-      const int r = h.level_rows[i], d = h.row_start[r + 1] - h.row_start[r];
+  for (int l = 0, e = 0; l < levels; l++) {
+    for (int i = sched.level_start[l]; i < sched.level_start[l + 1]; i++) {
+      const int r = sched.level_rows[i], d = h.row_start[r + 1] - h.row_start[r];
       for (int k = 0; k < d; k++, e++)
         tab[e] = (int32_t)((uint32_t)h.vars[h.row_start[r] + k] | (uint32_t)k << 16 | (uint32_t)d << 24);
       row.push_back(e);
@@ -197,7 +198,7 @@ cb_status ensure_edges(cb_ldpc* c, int max_level_edges, int slots, int warps) {
   d.n = h.n;
   d.m = h.m;
   d.edges = h.edges;
-  d.levels = h.levels;
+  d.levels = levels;
   d.max_level_edges = max_level_edges;
   d.warps = warps;
   d.edge = reinterpret_cast<const uint32_t*>(c->d_tables);
@@ -226,22 +227,26 @@ cb_status ensure_device(cb_ldpc* c) {
   // products as a scan does.
   c->edge_slots = 0;
   if (c->layered && c->rule == CB_RULE_SUM_PRODUCT && h.max_level_rows > 8) {
+    // a warp per 32 edges of the mean level, and the levels filled towards full warps: the
+    // FP64 pipe takes as long for a part of a warp as for all of it (PEG(576, 288): 77 -> 88 %
+    // of the lanes at work, PEG(1024, 512): 88 -> 97)
+    const int warps = std::min(cbk::kEdgeThreads / 32, std::max(1, (h.edges / std::max(1, h.levels) + 31) / 32));
+    const cbh::LevelSchedule sched = cbh::balanced_levels(h, 32 * warps);
+    const int levels = (int)sched.level_start.size() - 1;
     int max_level_edges = 0;
-    for (int l = 0; l < h.levels; l++) {
+    for (int l = 0; l < levels; l++) {
       int e = 0;
-      for (int i = h.level_start[l]; i < h.level_start[l + 1]; i++)
-        e += h.row_start[h.level_rows[i] + 1] - h.row_start[h.level_rows[i]];
+      for (int i = sched.level_start[l]; i < sched.level_start[l + 1]; i++)
+        e += h.row_start[sched.level_rows[i] + 1] - h.row_start[sched.level_rows[i]];
       max_level_edges = std::max(max_level_edges, e);
     }
     const int p = c->precision == CB_F64 ? 0 : 1;
     const size_t per = cbk::sparse_edges_slot_bytes(h.n, h.edges, max_level_edges, p);
-    const size_t tab = cbk::sparse_edges_table_bytes(h.edges, h.m, h.levels);
-    // a warp per 32 edges of the mean level
-    const int warps = std::min(cbk::kEdgeThreads / 32, std::max(1, (h.edges / std::max(1, h.levels) + 31) / 32));
+    const size_t tab = cbk::sparse_edges_table_bytes(h.edges, h.m, levels);
     const int slots = tab >= kEdgeSmem ? 0
                                        : (int)std::min<size_t>({(size_t)cbk::kEdgeMaxSlots, (kEdgeSmem - tab) / per,
                                                                 (size_t)(cbk::kEdgeThreads / (32 * warps))});
-    if (slots >= 1 && h.max_row_degree <= 255) return ensure_edges(c, max_level_edges, slots, warps);
+    if (slots >= 1 && h.max_row_degree <= 255) return ensure_edges(c, sched, max_level_edges, slots, warps);
   }
   // the launch shape decides the message layout: a thread per row with messages in
   // global memory takes the transposed one

@@ -13,9 +13,9 @@
 //     after a barrier, the product of the row's other tanh values and its own outgoing
 //     message.
 // Measured (GB300, f64, words with the copies): PEG(1024, 512), 4096 words of 13 iterations
-// 69 -> 31.5 ms; PEG(576, 288), 2000 words of 3 iterations, some of 50, 16.2 -> 5.6 ms; one
-// word of PEG(301, 150) 0.87 -> 0.24 ms.  f32 1.2-1.8 times faster.  The FP64 pipe is now
-// 75-80 % busy with 22-26 of 32 lanes at work: a level's last warp is part empty.
+// 69 -> 30 ms; PEG(576, 288), 2000 words of 3 iterations, some of 50, 16.9 -> 5.1 ms; one
+// word of PEG(301, 150) 0.87 -> 0.23 ms.  f32 1.3-1.9 times faster.  What is left is the
+// FP64 pipe, 75-80 % busy: about 67 instructions an edge (tanh 14 or 24, atanh 36).
 // The product is formed as check_row (sparse.cu) forms it: the running product of the
 // edges before, first to last, times that of the edges after, last to first, so the results
 // are the same bits.

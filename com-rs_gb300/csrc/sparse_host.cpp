@@ -83,6 +83,48 @@ bool build_sparse_code(int n, int m, const int32_t* row_start, const int32_t* va
   return true;
 }
 
+LevelSchedule balanced_levels(const SparseCode& c, int edges) {
+  // row r waits for the row before it of each of its variables
+  std::vector<std::vector<int32_t>> next(c.m);
+  std::vector<int32_t> waits(c.m, 0), last(c.n, -1), height(c.m, 1);
+  for (int r = 0; r < c.m; r++)
+    for (int e = c.row_start[r]; e < c.row_start[r + 1]; e++) {
+      int32_t& p = last[c.vars[e]];
+      if (p >= 0) {
+        next[p].push_back(r);
+        waits[r]++;
+      }
+      p = r;
+    }
+  for (int r = c.m - 1; r >= 0; r--)
+    for (int32_t s : next[r]) height[r] = std::max(height[r], height[s] + 1);
+  LevelSchedule out;
+  out.level_start.push_back(0);
+  std::vector<int32_t> ready, later;
+  for (int r = 0; r < c.m; r++)
+    if (waits[r] == 0) ready.push_back(r);
+  for (int left = c.levels; !ready.empty(); left--) {
+    std::stable_sort(ready.begin(), ready.end(), [&](int32_t a, int32_t b) { return height[a] > height[b]; });
+    later.clear();
+    int sum = 0;
+    for (int32_t r : ready) {
+      const int d = c.row_start[r + 1] - c.row_start[r];
+      if (height[r] >= left || sum == 0 || sum + d <= edges) {
+        sum += d;
+        out.level_rows.push_back(r);
+      } else {
+        later.push_back(r);
+      }
+    }
+    for (size_t i = out.level_start.back(); i < out.level_rows.size(); i++)
+      for (int32_t s : next[out.level_rows[i]])
+        if (--waits[s] == 0) later.push_back(s);
+    out.level_start.push_back((int32_t)out.level_rows.size());
+    ready.swap(later);
+  }
+  return out;
+}
+
 ChainBlocks chain_blocks(const SparseCode& c, int max_rows) {
   ChainBlocks out;
   out.linked.assign(c.m, 0);

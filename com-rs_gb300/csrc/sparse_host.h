@@ -34,6 +34,16 @@ struct SparseCode {
 bool build_sparse_code(int n, int m, const int32_t* row_start, const int32_t* vars, SparseCode& out,
                        std::string& err);
 
+// The layered schedule in as many levels as SparseCode's, each filled towards `edges`
+// edges: a row that the remaining levels' longest chain needs now is taken whatever the
+// sum, then the ready rows with the longest chains behind them as long as they fit.  Rows
+// that share a variable keep their order, as in SparseCode's schedule.
+struct LevelSchedule {
+  std::vector<int32_t> level_start;  // levels + 1
+  std::vector<int32_t> level_rows;   // m
+};
+LevelSchedule balanced_levels(const SparseCode& code, int edges);
+
 // Consecutive rows in blocks of at most max_rows: a row joins the block of the row before
 // it when it shares no variable with the block's rows, except that its second to last
 // variable may be the last one of the row before (a link: the accumulator of an IRA code).
