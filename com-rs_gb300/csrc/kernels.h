@@ -172,7 +172,7 @@ struct LearnedArgs {
   // f tape_frame + t tape_iter (tape_iter 0: each iteration's replace the one's before)
   unsigned char* tape;
   size_t tape_frame, tape_iter;
-  float* c2v;               // [n_frames][edges] the messages' gradients (backward)
+  float* c2v;               // [n_frames][entries][learned_stride] the messages' gradients (backward)
   float* post_out;          // [n_frames][n_full]
   float* loss;              // sum over frames of the mean bit loss (training)
   float* P;                 // [n_frames][T][n_full] posteriors after each iteration (multi-loss)
@@ -181,6 +181,9 @@ struct LearnedArgs {
   float* g_alpha;           // gradients of the mean loss (backward)
   float* g_beta;
 };
+// from one base-graph entry's message gradients to the next's: a compile-time constant of
+// the backward kernels
+inline int learned_stride(const cbd::DevCode& c) { return c.z <= 64 ? 64 : 384; }
 inline size_t learned_tape_bytes(const cbd::DevCode& c) { return (((size_t)c.rows_n * c.z * 12) + 15) & ~(size_t)15; }
 cudaError_t launch_learned(const LearnedArgs& a, bool forward, cudaStream_t stream);
 // codeword bytes [n_frames][n_bits] to packed words [n_frames][ceil(n_bits / 32)], LSB first

@@ -17,7 +17,7 @@
 // last iteration, or (multi-loss) a weighted mean over the outputs of all T iterations,
 // whose posteriors the forward then saves: weights 1/T, or a ramp 2(t+1)/(T(T+1)).
 // Backward: for t = T-1..0 and the layers in reverse, each row recomputes its forward
-// quantities from the saved inputs x and propagates
+// quantities from its saved record and propagates
 //   g_y = g_post[v] + g_c2v, g_a = g_y s [a > 0], dL/dalpha += g_a m, dL/dbeta -= g_a,
 //   g_m = g_a alpha flows to |x| of the argmin (or of the second argmin for the argmin),
 //   g_x = g_post[v] + sign(x) g_|x|, then g_post[v] = g_x and g_c2v = -g_x.
@@ -29,13 +29,14 @@
 // record where it kept the messages before: y follows from it and the previous iteration's
 // weights, the same bits.
 //
-// Bound: the latency of a frame's chain of rows (levels of one to three rows, a barrier
-// after each) at the residency that the posteriors allow, then issue.  Measured on GB300,
-// shared weights: 512 frames of BG1 Z = 384, 8 iterations, forward 3.57 -> 1.53 ms and
-// backward 6.52 -> 2.25 ms; 1024 frames of BG2 Z = 52, 10 iterations, 0.98 -> 0.48 and
-// 1.78 -> 0.79 ms (before: x on the tape, messages and weights read from global memory in
-// the rows, ten shuffles per edge for the weight gradients and their sums by shared-memory
-// atomics).
+// Bound: forward, issue (57-65 %); backward, the latency of the message gradients, 4 bytes
+// an edge read and written per iteration, of which BG1's resident frames hold 147 MB: more
+// than L2.  Measured on GB300, shared weights: 512 frames of BG1 Z = 384, 8 iterations,
+// forward 3.57 -> 1.43 ms and backward 6.52 -> 2.15 ms; 1024 frames of BG2 Z = 52, 10
+// iterations, 0.98 -> 0.46 and 1.78 -> 0.67 ms (before: x on the tape, messages and weights
+// read from global memory in the rows, ten shuffles per edge for the weight gradients and
+// their sums by shared-memory atomics).  Loading the next row's message gradients ahead, in
+// registers, measured 5-10 % slower.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -47,12 +48,11 @@ namespace cbk {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kMaxDegree = 19;
 // the edges of a level at most (the dense core rows of base graph 1)
 constexpr int kMaxLevelEdges = 19;
-// meta word: bits 0-4 the first edge of the smallest |x|, bits 5-9 that of the second
-// smallest, bits 10.. the signs (x < 0)
-constexpr int kMetaSigns = 10;
+// meta word: bits 0-4 the first edge of the smallest |x| (0 when that is infinite), bits
+// 5-9 that of the second smallest (likewise), bits 31, 30, .. the signs of x of edges 0, 1, ..
+constexpr uint32_t kMetaSigns = 0xffffe000u;
 
 // weight of iteration t's output in the multi-loss: 1/T each (mode 1), or a linear ramp
 // 2 (t + 1) / (T (T + 1)) that leans on the last iterations (mode 2)
@@ -75,7 +75,8 @@ struct Tape {
 __host__ __device__ inline size_t learned_post_bytes(int n_full) { return ((size_t)n_full * 4 + 15) & ~(size_t)15; }
 
 // The (scale, offset) of entry i for lifted row r in one iteration: shared weights staged
-// in shared memory as pairs, or one per lifted edge in global memory.
+// in shared memory as pairs, or one per lifted edge in global memory.  `none`: the iteration
+// before the first, whose scale 0 and offset +inf make every message 0.
 template <bool SHARED>
 struct RowWeights;
 template <>
@@ -86,58 +87,74 @@ struct RowWeights<true> {
 template <>
 struct RowWeights<false> {
   const float *al, *be;
+  bool none;
   __device__ __forceinline__ float2 at(int i, int z, int r) const {
     const size_t k = (size_t)i * z + r;
-    return make_float2(al[k], be[k]);
+    return none ? make_float2(0.f, INFINITY) : make_float2(al[k], be[k]);
   }
 };
 
-// the message of edge e from its row's record
-__device__ __forceinline__ float learned_message(float2 w, float m, uint32_t neg) {
-  const float am = __fmaf_rn(w.x, m, -w.y);
-  const float mag = am > 0.f ? am : 0.f;
-  return neg ? -mag : mag;
+// The magnitude max(alpha m - beta, 0) of a message.  A zero's sign is of no account: it is
+// added to or subtracted from posteriors that are never -0.0 (they start as 0.0 + LLR or 30.0).
+__device__ __forceinline__ float learned_mag(float2 w, float m) { return fmaxf(__fmaf_rn(w.x, m, -w.y), 0.f); }
+
+// bit 31 of a word of signs shifted left by an edge's number, on a value
+__device__ __forceinline__ float flip_sign(float v, uint32_t signs) {
+  return __uint_as_float(__float_as_uint(v) ^ (signs & 0x80000000u));
 }
 
-// forward of one lifted row, degree D, entries s0 ..; (o1, o2, om) the previous
-// iteration's record
+// forward of one lifted row, degree D, entries s0 ..; (o, om) the previous iteration's
+// record, wp and wc the previous and this iteration's weights
 template <int D, bool SHARED>
-__device__ __forceinline__ void learned_row_fwd(const LearnedArgs& a, float* post, int s0, int r, int z, bool first,
+__device__ __forceinline__ void learned_row_fwd(const LearnedArgs& a, float* post, int s0, int r, int z,
                                                 const RowWeights<SHARED>& wp, const RowWeights<SHARED>& wc, float2 o,
                                                 uint32_t om, float2& n, uint32_t& nm) {
   const EdgeAddrTable addr{a.code.eaddr + s0, r, 4 * r, 4 * z};
   int off[D];
   float x[D];
   const int oi1 = (int)(om & 31u);
-  const uint32_t os = om >> kMetaSigns, op = __popc(os) & 1u;
-  uint32_t sg = 0;
-  float m1 = INFINITY, m2 = INFINITY;
-  int i1 = 0, i2 = 0;
+  // the signs to add the old messages with: the opposite of the product of the others'
+  const uint32_t os = (__popc(om & kMetaSigns) & 1) ? om : ~om;
 #pragma unroll
   for (int e = 0; e < D; e++) {
     off[e] = addr(e);
-    float old = 0.f;
-    if (!first) old = learned_message(wp.at(s0 + e, z, r), e == oi1 ? o.y : o.x, op ^ ((os >> e) & 1u));
-    x[e] = __fsub_rn(ld_post(post, off[e]), old);
+    const float mag = learned_mag(wp.at(s0 + e, z, r), e == oi1 ? o.y : o.x);
+    x[e] = __fadd_rn(ld_post(post, off[e]), flip_sign(mag, os << e));
   }
+  // the two smallest magnitudes, two edges at a time (NaN counts as infinite)
+  float m1 = INFINITY, m2 = INFINITY;
+#pragma unroll
+  for (int e = 0; e + 1 < D; e += 2) {
+    const float p = fminf(fabsf(x[e]), INFINITY), q = fminf(fabsf(x[e + 1]), INFINITY);
+    const float lo = fminf(p, q);
+    m2 = min3f(m2, fmaxf(m1, lo), fmaxf(p, q));
+    m1 = fminf(m1, lo);
+  }
+  if (D & 1) {
+    const float p = fminf(fabsf(x[D - 1]), INFINITY);
+    m2 = fminf(m2, fmaxf(m1, p));
+    m1 = fminf(m1, p);
+  }
+  uint32_t sg = 0, at1 = 0, at2 = 0;
 #pragma unroll
   for (int e = 0; e < D; e++) {
-    sg |= (uint32_t)(x[e] < 0.f) << e;
-    const float av = fabsf(x[e]);
-    const bool lt1 = av < m1, lt2 = av < m2;
-    m2 = lt1 ? m1 : lt2 ? av : m2;
-    i2 = lt1 ? i1 : lt2 ? e : i2;
-    m1 = lt1 ? av : m1;
-    i1 = lt1 ? e : i1;
+    sg = __funnelshift_l(__float_as_uint(x[e]), sg, 1);
+    if (fabsf(x[e]) == m2) at2 |= 1u << e;
   }
-  const uint32_t par = __popc(sg) & 1u;
+  sg <<= 32 - D;
+  const uint32_t ns = (__popc(sg) & 1) ? ~sg : sg;  // the product of the other signs
 #pragma unroll
   for (int e = 0; e < D; e++) {
-    const float y = learned_message(wc.at(s0 + e, z, r), e == i1 ? m2 : m1, par ^ ((sg >> e) & 1u));
-    st_post(post, off[e], __fadd_rn(x[e], y));
+    const bool first = fabsf(x[e]) == m1;  // (on a tie m1 = m2)
+    if (first) at1 |= 1u << e;
+    const float mag = learned_mag(wc.at(s0 + e, z, r), first ? m2 : m1);
+    st_post(post, off[e], __fadd_rn(x[e], flip_sign(mag, ns << e)));
   }
+  // their first edges, as a scan with strict comparisons finds them
+  const uint32_t rest = m1 == m2 ? at1 & (at1 - 1) : at2;
+  const uint32_t i1 = m1 < INFINITY ? __ffs(at1) - 1 : 0, i2 = m2 < INFINITY ? __ffs(rest) - 1 : 0;
   n = make_float2(m1, m2);
-  nm = (uint32_t)i1 | (uint32_t)i2 << 5 | sg << kMetaSigns;
+  nm = i1 | i2 << 5 | sg;
 }
 
 // The sums of N values over the warp's lanes in about N + 5 shuffles: each step halves
@@ -176,61 +193,84 @@ struct WarpSums<N, 0> {
   static __device__ __forceinline__ int index(int j, int) { return j; }
 };
 
-// Backward of one lifted row from its record.  With shared weights `red` receives the
-// warp's sums of the gradients: D scales, then D offsets (every lane of the warp takes part;
-// the lanes without a row with zeros).
-template <int D, bool SHARED>
-__device__ __forceinline__ void learned_row_bwd(const LearnedArgs& a, float* gp, float* gc, float2 n, uint32_t nm,
+// the warp's sums of N values to red[0], red[1], ..
+template <int N>
+__device__ __forceinline__ void put_warp_sums(float (&v)[N], float* red, int lane) {
+  using Sums = WarpSums<N, 16>;
+  Sums::sum(v, lane);
+#pragma unroll
+  for (int j = 0; j < Sums::left; j++) {
+    const int i = Sums::index(j, lane);
+    if (i >= 0) red[i] = v[j];
+  }
+}
+
+// Backward of one lifted row from its record.  `gr` points at the row's message gradients,
+// S floats from edge to edge (a constant, so that their addresses are immediates).  With
+// shared weights `red` receives the warp's sums of the gradients: D scales, then D offsets with the
+// opposite sign (every lane of the warp takes part; the lanes without a row with zeros).
+template <int D, bool SHARED, int S>
+__device__ __forceinline__ void learned_row_bwd(const LearnedArgs& a, float* gp, float* gr, float2 n, uint32_t nm,
                                                 int t, int s0, int r, int z, bool active, bool last,
                                                 const RowWeights<SHARED>& w, float* red, int lane) {
-  float v[2 * D];  // the gradients of the scales, then of the offsets
-#pragma unroll
-  for (int i = 0; i < 2 * D; i++) v[i] = 0.f;
+  const int i1 = (int)(nm & 31u);
+  float ga[D];  // the gradients of max(alpha m - beta, 0): of the offsets, negated
   if (active) {
     const EdgeAddrTable addr{a.code.eaddr + s0, r, 4 * r, 4 * z};
     int off[D];
-    float gy[D];
-    const int i1 = (int)(nm & 31u), i2 = (int)((nm >> 5) & 31u);
-    const uint32_t sg = nm >> kMetaSigns, par = __popc(sg) & 1u;
+    int i2 = (int)((nm >> 5) & 31u);
+    const uint32_t sg = nm & kMetaSigns, ns = (__popc(sg) & 1) ? ~sg : sg;
 #pragma unroll
-    for (int e = 0; e < D; e++) gy[e] = last ? 0.f : gc[(size_t)(s0 + e) * z + r];
+    for (int e = 0; e < D; e++) ga[e] = last ? 0.f : gr[e * S];
     float g1 = 0.f, g2 = 0.f;  // gradients of |x_i1| and |x_i2|
 #pragma unroll
     for (int e = 0; e < D; e++) {
       off[e] = addr(e);
-      gy[e] = ld_post(gp, off[e]) + gy[e];
+      const float gy = ld_post(gp, off[e]) + ga[e];
       const float2 ab = w.at(s0 + e, z, r);
-      const float m = e == i1 ? n.y : n.x;
-      const float am = __fmaf_rn(ab.x, m, -ab.y);
-      const float g = (par ^ ((sg >> e) & 1u)) ? -gy[e] : gy[e];
-      const float ga = am > 0.f ? g : 0.f;
-      if constexpr (SHARED) {
-        v[e] = ga * m;
-        v[D + e] = -ga;
-      } else {
+      const bool min = e == i1;
+      const float m = min ? n.y : n.x;
+      ga[e] = __fmaf_rn(ab.x, m, -ab.y) > 0.f ? flip_sign(gy, ns << e) : 0.f;
+      if constexpr (!SHARED) {
         const size_t k = ((size_t)t * a.code.n_entries + s0 + e) * z + r;
-        atomicAdd(&a.g_alpha[k], ga * m);
-        atomicAdd(&a.g_beta[k], -ga);
+        atomicAdd(&a.g_alpha[k], ga[e] * m);
+        atomicAdd(&a.g_beta[k], -ga[e]);
       }
-      const float gm = ga * ab.x;
-      if (e == i1) g2 += gm;
+      const float gm = ga[e] * ab.x;
+      if (min) g2 = gm;
       else g1 += gm;
     }
+    // only the two smallest inputs' posteriors receive a gradient: x = post - c2v there
+    // adds sign(x) g_|x|, everywhere else the row leaves the posterior's gradient as it is
+    g1 = flip_sign(g1, sg << i1);
+    g2 = flip_sign(g2, sg << i2);
+    if (i2 == i1) i2 = 31;
 #pragma unroll
     for (int e = 0; e < D; e++) {
-      const float gabs = (e == i1 ? g1 : 0.f) + (e == i2 && i2 != i1 ? g2 : 0.f);
-      const float gx = ld_post(gp, off[e]) + (((sg >> e) & 1u) ? -gabs : gabs);
-      st_post(gp, off[e], gx);
-      if (t > 0) gc[(size_t)(s0 + e) * z + r] = -gx;
+      const bool at1 = e == i1, at2 = e == i2;
+      const float gx = ld_post(gp, off[e]) + (at1 ? g1 : at2 ? g2 : 0.f);
+      if (at1 || at2) st_post(gp, off[e], gx);
+      if (t > 0) gr[e * S] = -gx;
     }
+  } else {
+#pragma unroll
+    for (int e = 0; e < D; e++) ga[e] = 0.f;
   }
   if constexpr (SHARED) {
-    using S = WarpSums<2 * D, 16>;
-    S::sum(v, lane);
+    if constexpr (D <= 10) {
+      float v[2 * D];
 #pragma unroll
-    for (int j = 0; j < S::left; j++) {
-      const int i = S::index(j, lane);
-      if (i >= 0) red[i] = v[j];
+      for (int e = 0; e < D; e++) {
+        v[e] = ga[e] * (e == i1 ? n.y : n.x);
+        v[D + e] = ga[e];
+      }
+      put_warp_sums(v, red, lane);
+    } else {  // (two sums: 2 D values at once spill)
+      float v[D];
+#pragma unroll
+      for (int e = 0; e < D; e++) v[e] = ga[e] * (e == i1 ? n.y : n.x);
+      put_warp_sums(v, red, lane);
+      put_warp_sums(ga, red + D, lane);
     }
   }
 }
@@ -259,7 +299,7 @@ __device__ __forceinline__ RowWeights<SHARED> iteration_weights(const LearnedArg
     return {buf};
   } else {
     const size_t per = (size_t)ne * a.code.z;
-    return {a.alpha + t * per, a.beta + t * per};
+    return {a.alpha + t * per, a.beta + t * per, false};
   }
 }
 
@@ -298,12 +338,17 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
   const bool multi = a.multi_loss && a.P && a.cw_bits && a.loss;
   const bool active = tid < z;
   float lsum = 0.f;  // this thread's share of the loss
-  RowWeights<SHARED> wp = iteration_weights<SHARED>(a, wbuf, 0), wc = wp;
+  // before the first iteration there are no messages: weights that make them 0
+  RowWeights<SHARED> wp, wc;
+  if constexpr (SHARED) {
+    wc = {wbuf + ne};
+    for (int i = tid; i < ne; i += nt) wbuf[ne + i] = make_float2(0.f, INFINITY);
+  } else {
+    wc = {a.alpha, a.beta, true};
+  }
   for (int t = 0; t < a.T; t++) {
-    if (t > 0) {
-      wp = wc;
-      wc = iteration_weights<SHARED>(a, wbuf + (t & 1) * ne, t);
-    }
+    wp = wc;
+    wc = iteration_weights<SHARED>(a, wbuf + (t & 1) * ne, t);
     __syncthreads();
     const Tape old(tape + (t > 0 ? (size_t)(t - 1) * a.tape_iter : 0), lifted);
     const Tape cur(tape + (size_t)t * a.tape_iter, lifted);
@@ -328,7 +373,7 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
         const int s0 = c.layer_start[L], d = c.layer_start[L + 1] - s0;
         float2 n;
         uint32_t nm;
-#define CB_ROW(DD) learned_row_fwd<DD, SHARED>(a, post, s0, tid, z, t == 0, wp, wc, o, om, n, nm);
+#define CB_ROW(DD) learned_row_fwd<DD, SHARED>(a, post, s0, tid, z, wp, wc, o, om, n, nm);
         CB_LEARNED_DEGREES(CB_ROW)
 #undef CB_ROW
         cur.mag[L * z + tid] = n;
@@ -367,7 +412,7 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
   }
 }
 
-template <bool SHARED>
+template <bool SHARED, int S>
 __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_constant__ LearnedArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const cbd::DevCode& c = a.code;
@@ -380,8 +425,7 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
   constexpr int RW = 2 * kMaxLevelEdges;
   const long long f = blockIdx.x;
   if (f >= a.n_frames) return;
-  const size_t edges = (size_t)c.n_entries * z;
-  float* gc = a.c2v + (size_t)f * edges;  // the message gradients
+  float* gc = a.c2v + (size_t)f * c.n_entries * S + tid;  // this thread's message gradients
   const int wpc = (c.n_full + 31) >> 5;
   const bool multi = a.multi_loss && a.P;
   const bool active = tid < z;
@@ -395,10 +439,24 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
     if (multi || t == a.T - 1) {
       const float* p = multi ? a.P + ((size_t)f * a.T + t) * c.n_full : a.post_out + (size_t)f * c.n_full;
       const float sc = multi ? scale * iter_loss_weight(a.multi_loss, t, a.T) : scale;
-      for (int v = tid; v < a.loss_bits; v += nt) {
-        int bit = (a.cw_bits[(size_t)f * wpc + (v >> 5)] >> (v & 31)) & 1;
-        float sgn = bit ? -1.f : 1.f;
-        gp[v] += -sgn * sigmoid_f(-sgn * p[v]) * sc;
+      // eight posteriors in flight: one at a time, their latency was a third of the kernel
+      constexpr int U = 8;
+      for (int v0 = tid; v0 < a.loss_bits; v0 += U * nt) {
+        float q[U];
+        uint32_t cw[U];
+#pragma unroll
+        for (int j = 0; j < U; j++) {
+          const int v = v0 + j * nt;
+          q[j] = v < a.loss_bits ? p[v] : 0.f;
+          cw[j] = v < a.loss_bits ? a.cw_bits[(size_t)f * wpc + (v >> 5)] : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < U; j++) {
+          const int v = v0 + j * nt;
+          if (v >= a.loss_bits) break;
+          const float sgn = ((cw[j] >> (v & 31)) & 1) ? -1.f : 1.f;
+          gp[v] += -sgn * sigmoid_f(-sgn * q[j]) * sc;
+        }
       }
     }
     __syncthreads();
@@ -425,8 +483,8 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
           nmn = cur.meta[i];
         }
         float* rd = red + ((size_t)buf * nw + warp) * RW + 2 * at;
-#define CB_ROW(DD) \
-  learned_row_bwd<DD, SHARED>(a, gp, gc, n, nm, t, s0, tid, z, active, t == a.T - 1, w, rd, lane);
+#define CB_ROW(DD)                                                                                                 \
+  learned_row_bwd<DD, SHARED, S>(a, gp, gc + (size_t)s0 * S, n, nm, t, s0, tid, z, active, t == a.T - 1, w, rd, lane);
         CB_LEARNED_DEGREES(CB_ROW)
 #undef CB_ROW
         n = nn;
@@ -444,7 +502,7 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
             float s = 0.f;
             for (int k = 0; k < nw; k++) s += rd[k * RW];
             const size_t wi = (size_t)t * c.n_entries + s0 + (i < d ? i : i - d);
-            atomicAdd(i < d ? &a.g_alpha[wi] : &a.g_beta[wi], s);
+            atomicAdd(i < d ? &a.g_alpha[wi] : &a.g_beta[wi], i < d ? s : -s);
           }
           base += d;
         }
@@ -486,8 +544,14 @@ __global__ void adam_kernel(float* w, const float* g, float* m, float* v, int64_
 
 cudaError_t launch_learned(const LearnedArgs& a, bool forward, cudaStream_t s) {
   const int threads = ((a.code.z + 31) / 32) * 32;
-  void* k = forward ? (a.shared ? (void*)learned_forward_kernel<true> : (void*)learned_forward_kernel<false>)
-                    : (a.shared ? (void*)learned_backward_kernel<true> : (void*)learned_backward_kernel<false>);
+  void* k;
+  if (forward) {
+    k = a.shared ? (void*)learned_forward_kernel<true> : (void*)learned_forward_kernel<false>;
+  } else if (learned_stride(a.code) == 64) {
+    k = a.shared ? (void*)learned_backward_kernel<true, 64> : (void*)learned_backward_kernel<false, 64>;
+  } else {
+    k = a.shared ? (void*)learned_backward_kernel<true, 384> : (void*)learned_backward_kernel<false, 384>;
+  }
   size_t smem = learned_post_bytes(a.code.n_full);
   if (a.shared)
     smem += forward ? 2 * sizeof(float2) * a.code.n_entries
