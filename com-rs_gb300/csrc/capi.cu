@@ -191,6 +191,7 @@ cb_status decode_device_impl(cb_code* c, const T* llr, int64_t n, uint32_t* bits
   a.work_counter = reinterpret_cast<int32_t*>(c->d_counter);
   a.status = c->d_status;
   CB_CUDA(c, cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned long long), s));
+  a.full_grid = c->decode_grid;
   int grid = (int)std::min<int64_t>(c->decode_grid, n);
   CB_CUDA(c, cbk::launch_decode<T>(a, grid, s));
   return CB_OK;

@@ -55,16 +55,25 @@ __host__ __device__ __forceinline__ size_t decode_smem_bytes(int n_full, int z, 
 enum LearnedWeights { kPlain = 0, kWeightsGlobal = 1, kWeightsParam = 2, kWeightsShared = 3 };
 
 // One layered iteration of decode_body: the rows in schedule order, each row's state from
-// the previous iteration (L2-resident: loaded where it is used), a barrier after each level.
-template <typename T, int LW, int RULE>
+// the previous iteration (L2-resident), a barrier after each level.  The full f64 build loads
+// the next row's state before the row's update (4096 frames of BG2 Z = 52: 2.80 -> 2.76 ms).
+template <typename T, int LW, int RULE, int MAXD, bool FULL>
 __device__ __forceinline__ void decode_layers(const cbd::DevCode& c, T* post, const StateSlot<T>& st,
                                               const LearnedRowW& lw, int iter, int tid, int z, bool active,
-                                              T alpha) {
+                                              T alpha, const ScaleF64& scale) {
+  constexpr bool AHEAD = sizeof(T) == 8 && FULL;
+  T b1 = (T)0, b2 = (T)0;
+  uint32_t bt = 0;
+  if (AHEAD && iter > 1 && active) st.load(c.layer_order[0] * z + tid, b1, b2, bt);
   for (int q = 0; q < c.rows_n; q++) {
     const int L = c.layer_order[q];
-    T a1 = (T)0, a2 = (T)0;
-    uint32_t mt = 0;
-    if (iter > 1 && active) st.load(L * z + tid, a1, a2, mt);
+    T a1 = b1, a2 = b2;
+    uint32_t mt = bt;
+    if (AHEAD) {
+      if (iter > 1 && active && q + 1 < c.rows_n) st.load(c.layer_order[q + 1] * z + tid, b1, b2, bt);
+    } else if (iter > 1 && active) {
+      st.load(L * z + tid, a1, a2, mt);
+    }
     if (active) {
       const int s0 = c.layer_start[L];
       const int d = c.layer_start[L + 1] - s0;
@@ -78,14 +87,14 @@ __device__ __forceinline__ void decode_layers(const cbd::DevCode& c, T* post, co
         row_dispatch_lean<RULE>(d, post, EdgeAddrTable{c.eaddr + s0, tid, 4 * tid, 4 * z}, a1, a2, mt, alpha, n1, n2,
                                 nm);
       else
-        row_dispatch<T, RULE>(d, post, c.entry + s0, tid, z, a1, a2, mt, alpha, n1, n2, nm);
+        row_dispatch<RULE, MAXD, FULL>(d, post, c.entry + s0, tid, z, a1, a2, mt, scale, n1, n2, nm);
       st.store(L * z + tid, n1, n2, nm);
     }
     if (c.level_end[q]) __syncthreads();
   }
 }
 
-template <typename T, int LW>
+template <typename T, int LW, int MAXD, bool FULL>
 __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float* la, const float* lb) {
   constexpr bool LEARNED = LW != kPlain;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -102,6 +111,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float*
   const int rows = c.rows_n * z;
   const StateSlot<T> st(reinterpret_cast<unsigned char*>(a.state) + (size_t)blockIdx.x * slot_bytes<T>(rows), rows);
   const T alpha = (T)a.cfg.alpha;
+  const ScaleF64 scale = make_scale(a.cfg.alpha);  // f64
   const int rule = a.cfg.rule;
   const int max_it = a.cfg.max_iterations;
   const int wpf = (c.k_info + 31) >> 5;
@@ -191,9 +201,9 @@ __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float*
         // whole iteration, none in the rows)
         const LearnedRowW lw{w_ap, w_bp, w_ac, w_bc, 0, w_stride, w_roff};
         if (LEARNED || rule == cbd::RULE_NMS)
-          decode_layers<T, LW, cbd::RULE_NMS>(c, post, st, lw, iter, tid, z, active, alpha);
+          decode_layers<T, LW, cbd::RULE_NMS, MAXD, FULL>(c, post, st, lw, iter, tid, z, active, alpha, scale);
         else
-          decode_layers<T, LW, cbd::RULE_OMS>(c, post, st, lw, iter, tid, z, active, alpha);
+          decode_layers<T, LW, cbd::RULE_OMS, MAXD, FULL>(c, post, st, lw, iter, tid, z, active, alpha, scale);
         if (!some_check_fails(post, hd, s_ent, s_lstart, c.rows_n, ncol, z, tid, nt)) {
           it = iter;
           break;
@@ -250,21 +260,33 @@ __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float*
   }
 }
 
-template <typename T, int LW>
+template <typename T, int LW, int MAXD, bool FULL>
 __global__ void __launch_bounds__(384, sizeof(T) == 4 ? 2 : 1) layered_kernel(const __grid_constant__ DecodeArgs<T> a) {
-  decode_body<T, LW>(a, a.l_alpha, a.l_beta);
+  decode_body<T, LW, MAXD, FULL>(a, a.l_alpha, a.l_beta);
 }
 
 __global__ void __launch_bounds__(384, 2) layered_learned_param_kernel(const __grid_constant__ LearnedParamArgs a) {
-  decode_body<float, kWeightsParam>(a.d, a.alpha, a.beta);
+  decode_body<float, kWeightsParam, 19, true>(a.d, a.alpha, a.beta);
+}
+
+// The plain decoder.  f64 has four builds: codes without rows of more than 10 edges (base
+// graph 2: 126 registers instead of 148), and, when every SM has its CTAs, the scaling's
+// products on the integer pipes and the next row's state loaded ahead.  Those take the FP64
+// pipe's time, not the latency of a row, of which a codeword alone on an SM is made: with them 96
+// codewords of BG1 Z = 144 take 1-3 % longer, 4096 of BG2 Z = 52 8 % less.
+void* plain_kernel(int precision, int max_degree, bool full) {
+  if (precision == 1) return (void*)layered_kernel<float, kPlain, 19, true>;
+  if (max_degree <= 10)
+    return full ? (void*)layered_kernel<double, kPlain, 10, true> : (void*)layered_kernel<double, kPlain, 10, false>;
+  return full ? (void*)layered_kernel<double, kPlain, 19, true> : (void*)layered_kernel<double, kPlain, 19, false>;
 }
 
 template <typename T>
-void* kernel_for(const DecodeArgs<T>& a) {
+void* kernel_for(const DecodeArgs<T>& a, int grid) {
   if constexpr (sizeof(T) == 4) {
-    if (a.l_alpha) return a.l_smem ? (void*)layered_kernel<T, kWeightsShared> : (void*)layered_kernel<T, kWeightsGlobal>;
+    if (a.l_alpha) return a.l_smem ? (void*)layered_kernel<T, kWeightsShared, 19, true> : (void*)layered_kernel<T, kWeightsGlobal, 19, true>;
   }
-  return (void*)layered_kernel<T, kPlain>;
+  return plain_kernel(sizeof(T) == 8 ? 0 : 1, a.code.max_degree, grid >= a.full_grid);
 }
 
 int block_threads(int z) { return ((z + 31) / 32) * 32; }
@@ -282,7 +304,7 @@ size_t decode_state_bytes_per_slot(const cbd::DevCode& c, int precision) {
 }
 
 int decode_grid_size(const cbd::DevCode& c, int precision, int device) {
-  void* k = precision == 0 ? (void*)layered_kernel<double, kPlain> : (void*)layered_kernel<float, kPlain>;
+  void* k = plain_kernel(precision, c.max_degree, true);
   size_t smem = smem_bytes(c, precision);
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0, sms = 0;
@@ -294,7 +316,7 @@ int decode_grid_size(const cbd::DevCode& c, int precision, int device) {
 template <typename T>
 cudaError_t launch_decode(const DecodeArgs<T>& a, int grid, cudaStream_t stream) {
   const int precision = sizeof(T) == 8 ? 0 : 1;
-  void* k = kernel_for<T>(a);
+  void* k = kernel_for<T>(a, grid);
   size_t smem = smem_bytes(a.code, precision) + (a.l_smem ? (size_t)4 * 4 * a.code.n_entries : 0);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
