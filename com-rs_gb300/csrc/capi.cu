@@ -519,6 +519,7 @@ cb_status ensure_device(cb_code* c) {
       c->use_nr = true;
       c->decode_grid = g;
       cbk::fill_nr_args(h, c->nr_args);
+      c->nr_args.live = c->dev.rows_live;
       c->nr_args.map = c->d_map;
       c->nr_args.inv_start = c->d_inv_start;
       c->nr_args.inv_t = c->d_inv_t;
@@ -577,6 +578,7 @@ cb_status cb_code_create(const cb_code_desc* d, cb_code** out) {
   c->cfg.layered = d->layered;
   c->cfg.max_iterations = d->max_iterations;
   cbk::fill_dev_code(c->host, c->dev);
+  cbk::set_live_rows(c->dev, cbk::decoder_rows(c->host, d->alpha));
   if (d->rule == CB_RULE_SUM_PRODUCT || !d->layered) {
     // lifted row (L, r) holds, for the entries (j, s) of base row L in table order, the
     // variable j Z + (r + s) mod Z (nr/ldpc.rs:124-134)
@@ -832,6 +834,7 @@ struct cb_nms {
   // change (cb_nms_set_weights, a training step)
   std::vector<float> h_w;
   bool h_w_valid = false;
+  int live = 0;  // the base rows that evaluation with these weights runs
   float* d_g = nullptr;
   float* d_m = nullptr;
   float* d_v = nullptr;
@@ -913,17 +916,37 @@ int nms_nr_grid(cb_nms* h) {
   return h->nr_grid;
 }
 
+// The base rows that evaluation runs: as the plain decoder (cbh::live_rows) when the skipped
+// rows' messages are zero, max(alpha 0 - beta, 0), so no offset of theirs but the own
+// column's is negative.  Needs the host copy of the weights.
+int nms_live_rows(const cb_nms* h) {
+  const cbh::NrCode& c = h->code->host;
+  const int live = cbh::live_rows(c), ne = (int)c.entry_col.size();
+  const float* beta = h->h_w.data() + h->nw;
+  for (int t = 0; t < h->T; t++)
+    for (int L = live; L < c.rows_n; L++)
+      for (int e = c.layer_start[L]; e + 1 < c.layer_start[L + 1]; e++)
+        if (beta[(size_t)t * ne + e] < 0.f) return c.rows_n;
+  return live;
+}
+
 cb_status nms_param_weights(cb_nms* h, std::vector<float>& w, bool& in_params) {
   cb_code* c = h->code;
   in_params = nms_nr_grid(h) > 0 || (h->shared && h->nw <= cbk::kMaxParamWeights && c->dev.z >= 128);
-  if (!in_params) return CB_OK;
+  // (weights per lifted edge stay on the device: their decoder runs every row)
+  const bool prunable = h->shared && cbh::live_rows(c->host) < c->host.rows_n;
+  if (!in_params && !prunable) {
+    h->live = c->host.rows_n;
+    return CB_OK;
+  }
   if (!h->h_w_valid) {
     h->h_w.resize((size_t)2 * h->nw);
     CB_CUDA(c, cudaMemcpyAsync(h->h_w.data(), h->d_w, h->h_w.size() * 4, cudaMemcpyDeviceToHost, c->stream));
     CB_CUDA(c, cudaStreamSynchronize(c->stream));
+    h->live = prunable ? nms_live_rows(h) : c->host.rows_n;
     h->h_w_valid = true;
   }
-  w = h->h_w;
+  if (in_params) w = h->h_w;
   return CB_OK;
 }
 
@@ -934,6 +957,7 @@ cb_status nms_eval(cb_nms* h, const float* llr, int64_t n, const uint32_t* ref, 
   cb_code* c = h->code;
   cbk::DecodeArgs<float> a;
   a.code = c->dev;
+  cbk::set_live_rows(a.code, h->live);
   a.cfg = c->cfg;
   a.cfg.max_iterations = h->T;
   a.llr = llr;
@@ -958,6 +982,7 @@ cb_status nms_eval(cb_nms* h, const float* llr, int64_t n, const uint32_t* ref, 
     static thread_local cbn::NrLearnedArgs la;
     la.a = c->nr_args;
     la.a.max_iterations = h->T;
+    la.a.live = h->live;
     la.a.llr = llr;
     la.a.n_frames = n;
     la.a.bits_out = nullptr;
@@ -1316,6 +1341,7 @@ cb_status decode_noalloc_impl(cb_code* c, void* scratch, const T* llr, int64_t n
   if (use_nr) {
     cbn::NrArgs a;
     cbk::fill_nr_args(c->host, a);
+    a.live = c->dev.rows_live;
     a.max_iterations = c->cfg.max_iterations;
     a.rule = c->cfg.rule;
     a.alpha = (float)c->cfg.alpha;

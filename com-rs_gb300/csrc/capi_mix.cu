@@ -283,7 +283,10 @@ cb_status cb_mix_create(const cb_mix_item* items, int64_t n, uint64_t seed, uint
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
   m->dev_codes.resize(m->codes.size());
-  for (size_t i = 0; i < m->codes.size(); i++) cbk::fill_dev_code(m->codes[i], m->dev_codes[i]);
+  for (size_t i = 0; i < m->codes.size(); i++) {
+    cbk::fill_dev_code(m->codes[i], m->dev_codes[i]);
+    cbk::set_live_rows(m->dev_codes[i], cbk::decoder_rows(m->codes[i], (double)m->alpha));
+  }
   m->gen_smem = 0;
   for (auto& kv : config_id) {
     const cbh::NrCode& h = m->codes[kv.first.first];

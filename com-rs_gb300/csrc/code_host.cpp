@@ -306,4 +306,17 @@ GenTables gen_tables(int k_info, int e, int m, int bits_threads, int noise_threa
   return g;
 }
 
+int live_rows(const NrCode& h) {
+  std::vector<int> degree(h.cols_k + h.rows_n + 1, 0);
+  for (uint16_t c : h.entry_col) degree[c]++;
+  int live = h.rows_n;
+  for (; live > 4; live--) {
+    const int col = h.cols_k + live - 1;
+    // (the own column is the row's last entry, as the tables list them)
+    if (h.entry_col[h.layer_start[live] - 1] != col || degree[col] != 1) break;
+    if (h.inv_start[(size_t)(col + 1) * h.z] != h.inv_start[(size_t)col * h.z]) break;  // some bit is sent
+  }
+  return live;
+}
+
 }  // namespace cbh

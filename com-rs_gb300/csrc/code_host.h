@@ -53,6 +53,17 @@ struct NrCode {
 
 bool build_nr_code(const CodeSpec& spec, NrCode& out, std::string& err);
 
+// The base rows before the trailing ones whose own parity column (an extension column, in
+// no other row) is not sent at all.  The variables of such a column start at LLR 0, so in every
+// iteration its row sends them zero and, its smallest incoming magnitude being theirs, every
+// other variable a message of magnitude alpha 0 (or max(0 - offset, 0)) = 0: the row changes
+// nothing but its own column.  No later row is live, so the decoders skip these rows, and form
+// their own column's posteriors from the others' when a syndrome test needs them.  At rate
+// 1/2 that leaves 24 of base graph 1's 46 rows (210 of 316 entries) and 12 of base graph 2's
+// 42 (77 of 197); the uneven mix of rates 1/3 to 5/6 decodes 16384 codewords in 9.0 instead of
+// 17.4 ms, 4096 f64 frames of BG2 Z = 52 at rate 1/2 in 1.3 instead of 2.8 ms.
+int live_rows(const NrCode& h);
+
 // xoshiro256** jump-ahead: the polynomial x^n mod P(x), P the characteristic
 // polynomial of the generator's linear state transition (256 coefficients).
 struct JumpPoly {

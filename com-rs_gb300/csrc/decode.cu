@@ -65,12 +65,12 @@ __device__ __forceinline__ void decode_layers(const cbd::DevCode& c, T* post, co
   T b1 = (T)0, b2 = (T)0;
   uint32_t bt = 0;
   if (AHEAD && iter > 1 && active) st.load(c.layer_order[0] * z + tid, b1, b2, bt);
-  for (int q = 0; q < c.rows_n; q++) {
+  for (int q = 0; q < c.rows_run; q++) {
     const int L = c.layer_order[q];
     T a1 = b1, a2 = b2;
     uint32_t mt = bt;
     if (AHEAD) {
-      if (iter > 1 && active && q + 1 < c.rows_n) st.load(c.layer_order[q + 1] * z + tid, b1, b2, bt);
+      if (iter > 1 && active && q + 1 < c.rows_run) st.load(c.layer_order[q + 1] * z + tid, b1, b2, bt);
     } else if (iter > 1 && active) {
       st.load(L * z + tid, a1, a2, mt);
     }
@@ -199,15 +199,26 @@ __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float*
         }
         // the rows of one iteration, the rule a template parameter (one branch around the
         // whole iteration, none in the rows)
-        const LearnedRowW lw{w_ap, w_bp, w_ac, w_bc, 0, w_stride, w_roff};
+        const LearnedRowW lw{w_ap, w_bp, w_ac, w_bc, 0, w_stride, w_roff};  // (of this thread's row)
         if (LEARNED || rule == cbd::RULE_NMS)
           decode_layers<T, LW, cbd::RULE_NMS, MAXD, FULL>(c, post, st, lw, iter, tid, z, active, alpha, scale);
         else
           decode_layers<T, LW, cbd::RULE_OMS, MAXD, FULL>(c, post, st, lw, iter, tid, z, active, alpha, scale);
-        if (!some_check_fails(post, hd, s_ent, s_lstart, c.rows_n, ncol, z, tid, nt)) {
+        // the skipped rows' own columns (formed for the full syndrome test only)
+        auto own = [&]() {
+          if (c.rows_live == c.rows_n) return;
+          unsent_rows(post, s_ent, s_lstart, c.rows_live, c.rows_n, z, tid, nt,
+                      [w_ac, w_bc, w_stride, z, rule, alpha](int e, int r, T m) -> T {
+            if constexpr (LEARNED) return LearnedRowW::mag_at(w_ac, w_bc, w_stride == 1 ? e : e * z + r, m);
+            else return rule == cbd::RULE_NMS ? mul_rn(alpha, m) : (T)fmax(sub_rn(m, alpha), (T)0);
+          });
+          __syncthreads();
+        };
+        if (!some_check_fails_after(post, hd, s_ent, s_lstart, c.rows_n, ncol, z, tid, nt, own)) {
           it = iter;
           break;
         }
+        if (LEARNED && iter == max_it && a.post_out) own();  // (the whole word's posteriors go out)
       }
     }
 

@@ -165,10 +165,13 @@ __device__ __forceinline__ void row_update_lean(float* __restrict__ post, const 
 struct LearnedRowW {
   const float *a_prev, *b_prev, *a_cur, *b_cur;
   int s0, stride, roff;
-  __device__ __forceinline__ float mag(const float* al, const float* be, int e, float m) const {
-    const int i = (s0 + e) * stride + roff;
+  // by the weights' index
+  static __device__ __forceinline__ float mag_at(const float* al, const float* be, int i, float m) {
     const float am = __fmaf_rn(al[i], m, -be[i]);
     return am > 0.f ? am : 0.f;
+  }
+  __device__ __forceinline__ float mag(const float* al, const float* be, int e, float m) const {
+    return mag_at(al, be, (s0 + e) * stride + roff, m);
   }
 };
 

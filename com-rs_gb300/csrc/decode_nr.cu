@@ -145,7 +145,9 @@ std::string jit_source(const cbh::NrCode& h, bool learned, int rule) {
     << "  static constexpr bool fixed = true;\n  static constexpr int z = " << h.z << ";\n"
     << "  static constexpr int shift[" << h.entry_shift.size() << "] = {";
   for (size_t t = 0; t < h.entry_shift.size(); t++) s << (t ? ", " : "") << h.entry_shift[t];
-  s << "};\n  static constexpr int rule = " << (learned ? 1 : rule) << ";\n};\n}  // namespace cbn\n";
+  // a code that sends every parity column runs every row: no tests in its iteration
+  s << "};\n  static constexpr int rule = " << (learned ? 1 : rule) << ";\n  static constexpr bool prune = "
+    << (cbh::live_rows(h) < h.rows_n ? "true" : "false") << ";\n};\n}  // namespace cbn\n";
   const char* P = learned ? "cbn::NrLearnedArgs" : "cbn::NrArgs";
   s << "template __global__ void cbn::layered_nr_kernel<" << h.bg << ", cbn::FixedLifting, " << P
     << ">(const __grid_constant__ " << P << ");\n";
@@ -330,6 +332,7 @@ void fill_nr_args(const cbh::NrCode& h, cbn::NrArgs& a) {
   a.k_info = h.k_info;
   a.e = h.e;
   a.rows = h.rows_n;
+  a.live = h.rows_n;
   a.n_entries = (int)h.entry_col.size();
   a.map_kind = h.map_is_offset ? 0 : (h.has_repeats ? 2 : 1);
   for (int t = 0; t < a.n_entries; t++) {

@@ -1,6 +1,7 @@
 // The device descriptor of a host-built NR code (host code shared by the ABI files).
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -55,6 +56,23 @@ inline void fill_dev_code(const cbh::NrCode& h, cbd::DevCode& v) {
   for (int t = 0; t < v.n_core_terms; t++)
     v.core_term[t] = ((uint32_t)h.core_terms[t].block << 20) | ((uint32_t)h.core_terms[t].src << 16) |
                      h.core_terms[t].shift;
+  v.rows_live = v.rows_run = h.rows_n;
+}
+
+// the base rows that a min-sum decoder runs: with a scale or offset that is negative or not
+// finite none is skipped
+inline int decoder_rows(const cbh::NrCode& h, double alpha) {
+  return alpha >= 0 && std::isfinite(alpha) ? cbh::live_rows(h) : h.rows_n;
+}
+
+// the schedule of the rows before `live`: whole levels
+inline void set_live_rows(cbd::DevCode& v, int live) {
+  v.rows_live = live;
+  int last = 0;  // the last position of a live row
+  for (int q = 0; q < v.rows_n; q++)
+    if (v.layer_order[q] < live) last = q;
+  while (!v.level_end[last]) last++;
+  v.rows_run = last + 1;
 }
 
 // the row degrees the decoders are compiled for (3..10 and 19)

@@ -113,16 +113,11 @@ __device__ __forceinline__ bool some_packed_check_fails(const T* post, uint32_t*
   return __syncthreads_or(bad) != 0;
 }
 
-// Whether some check fails on the hard decisions of post (hard_decisions_are_a_codeword,
-// ldpc.rs:555-557).  Block-wide.  Stage 1 reads the rows of the first two layers
-// directly (each thread its own row, stopping at the first failure): while the
-// decoder has not converged this almost always finds a failing check.  Only when every
-// one of those rows is satisfied does stage 2 test all rows on packed hard decisions.
-// Either way the answer is exactly "H c != 0".
+// Stage 1 of the syndrome test: the rows of the first two layers, read directly (each thread its
+// own row, stopping at the first failure).  Block-wide.
 template <typename T>
-__device__ __forceinline__ bool some_check_fails(const T* post, uint32_t* hd, const uint32_t* ent,
-                                                 const uint16_t* lstart, int rows_n, int ncol, int z, int tid,
-                                                 int nt) {
+__device__ __forceinline__ bool first_rows_fail(const T* post, const uint32_t* ent, const uint16_t* lstart, int z,
+                                                int tid) {
   int bad = 0;
   if (tid < z) {
     for (int L = 0; L < 2 && !bad; L++) {
@@ -136,8 +131,66 @@ __device__ __forceinline__ bool some_check_fails(const T* post, uint32_t* hd, co
       bad = (int)par;
     }
   }
-  if (__syncthreads_or(bad)) return true;
+  return __syncthreads_or(bad) != 0;
+}
+
+// Whether some check fails on the hard decisions of post (hard_decisions_are_a_codeword,
+// ldpc.rs:555-557).  Block-wide.  While the decoder has not converged stage 1 almost always
+// finds a failing check.  Only when every one of its rows is satisfied does stage 2 test all
+// rows on packed hard decisions.  Either way the answer is exactly "H c != 0".
+template <typename T>
+__device__ __forceinline__ bool some_check_fails(const T* post, uint32_t* hd, const uint32_t* ent,
+                                                 const uint16_t* lstart, int rows_n, int ncol, int z, int tid,
+                                                 int nt) {
+  if (first_rows_fail(post, ent, lstart, z, tid)) return true;
   return some_packed_check_fails(post, hd, ent, lstart, rows_n, ncol, z, tid, nt);
+}
+
+// some_check_fails after an iteration: `own` forms the own columns of skipped rows (see
+// unsent_rows) before stage 2 reads them
+template <typename T, class Own>
+__device__ __forceinline__ bool some_check_fails_after(const T* post, uint32_t* hd, const uint32_t* ent,
+                                                       const uint16_t* lstart, int rows_n, int ncol, int z, int tid,
+                                                       int nt, const Own& own) {
+  if (first_rows_fail(post, ent, lstart, z, tid)) return true;
+  own();
+  return some_packed_check_fails(post, hd, ent, lstart, rows_n, ncol, z, tid, nt);
+}
+
+// The own parity columns of the base rows [live, rows): columns that are not sent and in no
+// other row (cbh::live_rows).  What such a row makes of its variable is 0 + the message
+// from the row's other variables, whose messages from the row are zero: their smallest
+// magnitude through `mag` (the rule; entry of the own column, lifted row, magnitude) with the
+// product of their signs.  The own column is the row's last entry.
+template <typename T, class Mag>
+__device__ __forceinline__ void unsent_rows(T* post, const uint32_t* ent, const uint16_t* lstart, int live, int rows,
+                                            int z, int tid, int nt, const Mag mag) {
+  for (int task = tid; task < (rows - live) * z; task += nt) {
+    const int q = task / z, r = task - q * z, own = lstart[live + q + 1] - 1;
+    T m = infinity<T>();
+    uint32_t neg = 0;
+    for (int t = lstart[live + q]; t < own; t++) {
+      const uint32_t en = ent[t];
+      int cc = r + (int)(en & 0xffffu);
+      cc -= (cc >= z) ? z : 0;
+      const T v = post[(int)(en >> 16) * z + cc];
+      neg ^= (uint32_t)(v < (T)0);
+      m = fmin(m, fabs(v));
+    }
+    const uint32_t en = ent[own];
+    int cc = r + (int)(en & 0xffffu);
+    cc -= (cc >= z) ? z : 0;
+    const T o = mag(own, r, m);
+    post[(int)(en >> 16) * z + cc] = add_rn((T)0, neg ? -o : o);
+  }
+}
+
+// the same out of line: called once a codeword, and inlined its registers made the iteration of
+// the graph-specialised decoder spill
+template <typename T, class Mag>
+__device__ __noinline__ void unsent_rows_call(T* post, const uint32_t* ent, const uint16_t* lstart, int live, int rows,
+                                              int z, int tid, int nt, const Mag mag) {
+  unsent_rows(post, ent, lstart, live, rows, z, tid, nt, mag);
 }
 
 __device__ __forceinline__ float ld_post(const float* post, int off) {

@@ -52,6 +52,10 @@ struct DevCode {
   // no column, so their lifted rows run at once with the sequential order's results)
   uint8_t layer_order[cbh::kMaxLayers];
   uint8_t level_end[cbh::kMaxLayers];
+  // the decoders' rows (cbh::live_rows): rows from rows_live on change only their own column;
+  // rows_run positions of layer_order, whole levels, hold all the others (both rows_n when
+  // no row may be skipped)
+  int32_t rows_live, rows_run;
 };
 
 // decoder settings (crates/com-fec/src/ldpc.rs:165-172)

@@ -263,10 +263,10 @@ __device__ __forceinline__ void gen_one(const cbd::DevCode& c, const GenFrame<T>
   }
 }
 
-// (f64: four CTAs on an SM, 128 registers: the FP64 work of one covers the jumps, the encoding
+// (f32: five CTAs on an SM, 96 registers; f64: four, 128: the FP64 work of one covers the jumps, the encoding
 // and the power sum of the others; 4096 BG2 Z = 52 QPSK frames 1.30 -> 1.22 ms)
 template <typename T>
-__global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 4 : 1) gen_kernel(const __grid_constant__ GenArgs<T> a) {
+__global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 4 : 5) gen_kernel(const __grid_constant__ GenArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const long long frame = (long long)blockIdx.x;
   if (frame >= a.n_frames) return;

@@ -53,7 +53,7 @@ struct NrArgs {
   int32_t max_iterations;
   int32_t rule;              // 1: normalised min-sum, 2: offset min-sum
   float alpha;               // the scale or the offset
-  int32_t reserved;
+  int32_t live;              // the base rows before those that change only their own column (cbh::live_rows)
   const float* llr;          // [n_frames][E]
   int64_t n_frames;
   uint32_t* bits_out;        // [n_frames][ceil(K'/32)] (optional)
@@ -100,7 +100,7 @@ struct NrLearnedArgs {
 // the old messages), indexed by entry, as (scale, offset) pairs in shared memory.
 struct NrNoWeights {
   static constexpr bool learned = false;
-};
+};  // (the own columns of skipped rows take the rule's magnitude)
 struct NrRowWeights {
   static constexpr bool learned = true;
   const float2 *prev, *cur;
@@ -112,6 +112,7 @@ struct NrRowWeights {
 struct NrNoWeightSet {
   static constexpr bool learned = false;
   __device__ __forceinline__ NrNoWeights at(int) const { return {}; }
+  __device__ __forceinline__ NrNoWeights staged(int) const { return {}; }
 };
 // The weight rows [T + 1][entries] of the launch parameters: row t + 1 holds iteration
 // t's, row 0 the scale 0 and the offset +inf, whose magnitude max(0 m - inf, 0) is 0 for
@@ -138,6 +139,10 @@ struct NrParamWeightSet {
     __syncthreads();
     return {buf + (t & 1) * ne, cur};
   }
+  // the weights that at(t) staged
+  __device__ __forceinline__ NrRowWeights staged(int t) const {
+    return {buf + (t & 1) * ne, buf + ((t + 1) & 1) * ne};
+  }
 };
 
 // shared memory of the learned kernel: the plain decoder's and the two weight buffers
@@ -151,6 +156,7 @@ struct RuntimeLifting {
   static constexpr int z = 0;
   static constexpr int shift[1] = {0};
   static constexpr int rule = 0;  // the min-sum rule from the launch parameters
+  static constexpr bool prune = true;  // rows from a.live on are skipped
 };
 
 // How many rows ahead of its update a row's check-node state is loaded (0: at the row's
@@ -335,6 +341,14 @@ __device__ __forceinline__ void nr_row_learned(unsigned char* post, const NrArgs
   nr_row_learned_at<D>(post, off, S0, w, a1, a2, mt, n1, n2, nm);
 }
 
+// the lowest row from schedule position q on
+template <int BG>
+constexpr int rest_min(int q) {
+  int m = Graph<BG>::rows;
+  for (; q < Graph<BG>::rows; q++) m = Graph<BG>::order[q] < m ? Graph<BG>::order[q] : m;
+  return m;
+}
+
 struct NrState {
   unsigned char* mag;
   unsigned char* meta;
@@ -394,6 +408,13 @@ __device__ __forceinline__ void nr_iteration(unsigned char* post, const NrArgs& 
                                              int z4, int z, bool active, bool first, float alpha, const W& w,
                                              float a1, float a2, uint32_t mt, float b1, float b2, uint32_t bt) {
   if constexpr (Q < Graph<BG>::rows) {
+    // at a level's start: every row from here on changes only its own column, which is not
+    // sent (the syndrome test forms it)
+    if constexpr (K::prune && Q >= 4) {
+      if constexpr (Graph<BG>::level_end[Q - 1] != 0) {
+        if (a.live <= rest_min<BG>(Q)) return;
+      }
+    }
     constexpr int L = Graph<BG>::order[Q];
     constexpr int S0 = Graph<BG>::start[L];
     constexpr int D = Graph<BG>::start[L + 1] - S0;
@@ -438,13 +459,13 @@ __device__ __forceinline__ uint32_t row_parity(const unsigned char* post, const 
   }
 }
 
-// some_check_fails (dev_math.cuh) with stage 1, the rows of the first two base rows, at
+// some_check_fails_after (dev_math.cuh) with stage 1, the rows of the first two base rows, at
 // compile time: the same answer, exactly "H c != 0" (C2 on GB300, runtime lifting: 18.2
-// against 18.6 ms per 8192 codewords)
-template <int BG, class K>
+// against 18.6 ms per 8192 codewords).  `own` forms the skipped rows' own columns.
+template <int BG, class K, class Own>
 __device__ __forceinline__ bool some_nr_check_fails(const float* post, uint32_t* hd, const uint32_t* ent,
                                                     const uint16_t* lstart, const NrArgs& a, int ncol, int z, int tid,
-                                                    int nt, int r4, int z4) {
+                                                    int nt, int r4, int z4, const Own& own) {
   int bad = 0;
   if (tid < z) {
     int rr = tid, rr4 = r4;
@@ -454,6 +475,7 @@ __device__ __forceinline__ bool some_nr_check_fails(const float* post, uint32_t*
     if (!bad) bad = (int)row_parity<BG, K, Graph<BG>::start[1], Graph<BG>::start[2]>(p, a, rr, rr4, z4);
   }
   if (__syncthreads_or(bad)) return true;
+  if constexpr (K::prune) own();
   return some_packed_check_fails(post, hd, ent, lstart, a.rows, ncol, z, tid, nt);
 }
 
@@ -503,6 +525,17 @@ __global__ void __launch_bounds__(384, 2) layered_nr_kernel(const __grid_constan
   const int r4 = 4 * tid, z4 = 4 * z;
   for (int i = tid; i < a.n_entries; i += nt) s_ent[i] = a.entry[i];
   for (int i = tid; i <= a.rows; i += nt) s_lstart[i] = a.layer_start[i];
+
+  // the posteriors of the skipped rows' own columns after iteration `iter`
+  auto own_columns = [&](int iter) {
+    if (a.live == a.rows) return;
+    const auto w = wset.staged(iter - 1);
+    unsent_rows_call(post, s_ent, s_lstart, a.live, a.rows, z, tid, nt, [w, nms, alpha](int e, int, float m) {
+      if constexpr (decltype(w)::learned) return learned_mag(w.ac(e), w.bc(e), m);
+      else return nms ? __fmul_rn(alpha, m) : fmaxf(__fsub_rn(m, alpha), 0.0f);
+    });
+    __syncthreads();
+  };
 
   for (;;) {
     if (tid == 0) {
@@ -593,11 +626,16 @@ __global__ void __launch_bounds__(384, 2) layered_nr_kernel(const __grid_constan
                                     b1, b2, bt);
         }
         }
-        if (!some_nr_check_fails<BG, K>(post, hd, s_ent, s_lstart, a, ncol, z, tid, nt, r4, z4)) {
+        if (!some_nr_check_fails<BG, K>(post, hd, s_ent, s_lstart, a, ncol, z, tid, nt, r4, z4,
+                                        [&] { own_columns(iter); })) {
           it = iter;
           break;
         }
       }
+    }
+    // (a word that stopped has them already)
+    if constexpr (K::prune && decltype(wset)::learned) {
+      if (post_out && it == max_it && it > 0) own_columns(it);
     }
 
     // ---- outputs: hard decisions (signal.rs:47-49), counts (errors.rs:39-42); the decision

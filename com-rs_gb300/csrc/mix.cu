@@ -32,8 +32,10 @@ __device__ __forceinline__ bool slot_any(int bad, int* flag, int bar, int n, int
 
 // Whether some check fails, for one slot: stage 1 on the rows of the first two
 // layers, stage 2 on packed hard decisions (the test of decode.cu's some_check_fails).
+// `own` forms the own columns of skipped rows before stage 2 reads them.
+template <class Own>
 __device__ bool slot_check_fails(const float* post, uint32_t* hd, const uint32_t* ent, const uint16_t* lstart,
-                                 int rows_n, int ncol, int z, int lt, int nt, int bar, int* flag) {
+                                 int rows_n, int ncol, int z, int lt, int nt, int bar, int* flag, const Own& own) {
   int bad = 0;
   for (int r = lt; r < z && !bad; r += nt)
     for (int L = 0; L < 2 && !bad; L++) {
@@ -47,6 +49,7 @@ __device__ bool slot_check_fails(const float* post, uint32_t* hd, const uint32_t
       bad = (int)par;
     }
   if (slot_any(bad, flag, bar, nt, lt)) return true;
+  own();
   build_hard_decisions(post, hd, ncol, z, lt, nt);
   slot_sync(bar, nt);
   const int wz = (z + 31) >> 5, ws = wz + 1;
@@ -102,13 +105,15 @@ __device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned 
   for (int v = c.k_info + lt; v < c.k; v += nt) post[v] = cbd::kKnownBitLlr;
   slot_sync(bar, nt);
   int iters = 0;
-  const int rows_n = c.rows_n;
-  if (slot_check_fails(post, hd, s_ent, s_lstart, rows_n, ncol, z, lt, nt, bar, flag)) {
+  const int rule = a.rule;
+  const float alpha = a.alpha;
+  const int rows_n = c.rows_n, rows_run = c.rows_run, rows_live = c.rows_live;
+  if (slot_check_fails(post, hd, s_ent, s_lstart, rows_n, ncol, z, lt, nt, bar, flag, [] {})) {
     iters = a.max_it;
     for (int iter = 1; iter <= a.max_it; iter++) {
       // the base rows by levels, as decode.cu runs them; each row's state is loaded where
       // it is used (loaded one row ahead: 17.56 against 17.40 ms per decode phase)
-      for (int k = 0; k < rows_n; k++) {
+      for (int k = 0; k < rows_run; k++) {
         const int L = s_order[k];
         const int s0 = s_lstart[L], d = s_lstart[L + 1] - s0;
 #pragma unroll
@@ -129,7 +134,14 @@ __device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned 
         }
         if (s_end[k]) slot_sync(bar, nt);
       }
-      if (!slot_check_fails(post, hd, s_ent, s_lstart, rows_n, ncol, z, lt, nt, bar, flag)) {
+      auto own = [&]() {
+        if (rows_live == rows_n) return;
+        unsent_rows(post, s_ent, s_lstart, rows_live, rows_n, z, lt, nt, [rule, alpha](int, int, float m) {
+          return rule == cbd::RULE_NMS ? __fmul_rn(alpha, m) : fmaxf(__fsub_rn(m, alpha), 0.f);
+        });
+        slot_sync(bar, nt);
+      };
+      if (!slot_check_fails(post, hd, s_ent, s_lstart, rows_n, ncol, z, lt, nt, bar, flag, own)) {
         iters = iter;
         break;
       }
