@@ -343,7 +343,7 @@ __device__ __forceinline__ void nr_row_learned(unsigned char* post, const NrArgs
 
 // the lowest row from schedule position q on
 template <int BG>
-constexpr int rest_min(int q) {
+__host__ __device__ constexpr int rest_min(int q) {
   int m = Graph<BG>::rows;
   for (; q < Graph<BG>::rows; q++) m = Graph<BG>::order[q] < m ? Graph<BG>::order[q] : m;
   return m;
