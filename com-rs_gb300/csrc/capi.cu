@@ -1020,6 +1020,8 @@ cb_status nms_eval(cb_nms* h, const float* llr, int64_t n, const uint32_t* ref, 
 cbk::LearnedArgs nms_args(cb_nms* h, int64_t n) {
   cbk::LearnedArgs a{};
   a.code = h->code->dev;
+  cbk::set_live_rows(a.code, cbh::live_rows(h->code->host));
+  a.live = reinterpret_cast<int32_t*>(h->d_loss) + 1;
   a.T = h->T;
   a.shared = h->shared;
   a.alpha = h->d_w;

@@ -181,6 +181,7 @@ struct LearnedArgs {
   int32_t loss_bits;        // the loss covers codeword bits [0, loss_bits): n_full, or K' (the information bits)
   float* g_alpha;           // gradients of the mean loss (backward)
   float* g_beta;
+  int32_t* live;            // shared weights: the rows that the passes run, set by the forward launch
 };
 // from one base-graph entry's message gradients to the next's: a compile-time constant of
 // the backward kernels

@@ -29,14 +29,24 @@
 // record where it kept the messages before: y follows from it and the previous iteration's
 // weights, the same bits.
 //
+// Rows from c.rows_live on (cbh::live_rows: their own parity column is not sent and in no
+// other row) send the other variables zero while their offsets are not negative, which
+// learned_live_kernel tests before each pass over the frames.  Such a row is then only what
+// it makes of its own column, m the smallest |post| of its other variables:
+//   post_own = s max(alpha m - beta, 0),
+// and backward the gradient of post_own's own loss, through alpha m, onto m's variable.  Its
+// record is m, m's variable and two signs.  (Half of base graph 1's rows at rate 1/2, three
+// quarters of base graph 2's: 61 % of its edges.)
+//
 // Bound: forward, issue (57-65 %); backward, the latency of the message gradients, 4 bytes
-// an edge read and written per iteration, of which BG1's resident frames hold 147 MB: more
-// than L2.  Measured on GB300, shared weights: 512 frames of BG1 Z = 384, 8 iterations,
-// forward 3.57 -> 1.43 ms and backward 6.52 -> 2.15 ms; 1024 frames of BG2 Z = 52, 10
-// iterations, 0.98 -> 0.46 and 1.78 -> 0.67 ms (before: x on the tape, messages and weights
-// read from global memory in the rows, ten shuffles per edge for the weight gradients and
-// their sums by shared-memory atomics).  Loading the next row's message gradients ahead, in
-// registers, measured 5-10 % slower.
+// an edge read and written per iteration, more than L2 holds for BG1's resident frames.
+// Measured on GB300, shared weights: a step of 512 frames of BG1 Z = 384, 8 iterations, 10.3
+// -> 3.2 ms (forward 3.57, backward 6.52 before; 1.43 and 2.15 with every row run); 1024
+// frames of BG2 Z = 52, 10 iterations, forward 0.98 -> 0.36 ms (0.46 with every row) and
+// backward 1.78 -> 0.44 (0.67).  Before: x on the tape, messages and weights read from global memory
+// in the rows, ten shuffles per edge for the weight gradients and their sums by shared-memory
+// atomics.  Loading the next row's message gradients ahead, in registers, measured 5-10 %
+// slower.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -50,6 +60,7 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 // the edges of a level at most (the dense core rows of base graph 1)
 constexpr int kMaxLevelEdges = 19;
+constexpr int kOwnGroup = 8;  // skipped rows whose gradients are summed together
 // meta word: bits 0-4 the first edge of the smallest |x| (0 when that is infinite), bits
 // 5-9 that of the second smallest (likewise), bits 31, 30, .. the signs of x of edges 0, 1, ..
 constexpr uint32_t kMetaSigns = 0xffffe000u;
@@ -275,6 +286,48 @@ __device__ __forceinline__ void learned_row_bwd(const LearnedArgs& a, float* gp,
   }
 }
 
+// forward of one row that only makes its own column: lifted row r of entries [s0, s0 + d), own = the
+// last one, with its weights w
+__device__ __forceinline__ void own_column_fwd(const LearnedArgs& a, float* post, int s0, int d, int r, int z, float2 w,
+                                               float2& n, uint32_t& nm) {
+  const EdgeAddrTable addr{a.code.eaddr + s0, r, 4 * r, 4 * z};
+  float m = INFINITY;
+  int at = addr(0);
+  uint32_t neg = 0, neg_at = 0;
+  for (int e = 0; e + 1 < d; e++) {
+    const int o = addr(e);
+    const float x = ld_post(post, o), av = fabsf(x);
+    const uint32_t s = x < 0.f;
+    neg ^= s;
+    if (av < m || e == 0) neg_at = s;
+    if (av < m) {
+      m = av;
+      at = o;
+    }
+  }
+  const float y = learned_mag(w, m);
+  st_post(post, addr(d - 1), __fadd_rn(0.f, neg ? -y : y));
+  n = make_float2(__int_as_float(at), m);
+  nm = neg | neg_at << 1;
+}
+
+// *live: the rows that a pass with shared weights runs: c.rows_live, or all when a skipped row
+// has a negative offset on another edge than its own column's
+__global__ void __launch_bounds__(256) learned_live_kernel(const __grid_constant__ LearnedArgs a) {
+  const cbd::DevCode& c = a.code;
+  const int first = c.layer_start[c.rows_live], count = c.n_entries - first;
+  int bad = 0;
+  for (int i = threadIdx.x; i < a.T * count; i += blockDim.x) {
+    const int t = i / count, e = first + i - t * count;
+    if (!(a.beta[(size_t)t * c.n_entries + e] < 0.f)) continue;
+    bool own = false;
+    for (int L = c.rows_live; L < c.rows_n; L++) own = own || e + 1 == c.layer_start[L + 1];
+    if (!own) bad = 1;
+  }
+  bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) *a.live = bad ? c.rows_n : c.rows_live;
+}
+
 #define CB_LEARNED_DEGREES(ROW) \
   switch (d) {                  \
     case 3: ROW(3) break;       \
@@ -337,6 +390,7 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
   __syncthreads();
   const bool multi = a.multi_loss && a.P && a.cw_bits && a.loss;
   const bool active = tid < z;
+  const int live = SHARED ? *a.live : c.rows_n, run = live < c.rows_n ? c.rows_run : c.rows_n;
   float lsum = 0.f;  // this thread's share of the loss
   // before the first iteration there are no messages: weights that make them 0
   RowWeights<SHARED> wp, wc;
@@ -360,16 +414,16 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
       o = old.mag[i];
       om = old.meta[i];
     }
-    for (int q = 0; q < c.rows_n; q++) {
+    for (int q = 0; q < run; q++) {
       const int L = c.layer_order[q];
       float2 on = o;
       uint32_t omn = om;
-      if (active && t > 0 && q + 1 < c.rows_n) {
+      if (active && t > 0 && q + 1 < run) {
         const int i = c.layer_order[q + 1] * z + tid;
         on = old.mag[i];
         omn = old.meta[i];
       }
-      if (active) {
+      if (active && L < live) {  // (a skipped row may share the last live level)
         const int s0 = c.layer_start[L], d = c.layer_start[L + 1] - s0;
         float2 n;
         uint32_t nm;
@@ -382,6 +436,20 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
       o = on;
       om = omn;
       if (c.level_end[q]) __syncthreads();
+    }
+    // the skipped rows' own columns, where the loss or the output reads them
+    if (SHARED && live < c.rows_n && (t == a.T - 1 || (multi && a.loss_bits > (c.cols_k + live) * z))) {
+      if (active) {
+        for (int L = live; L < c.rows_n; L++) {
+          const int s0 = c.layer_start[L], s1 = c.layer_start[L + 1];
+          float2 n;
+          uint32_t nm;
+          own_column_fwd(a, post, s0, s1 - s0, tid, z, wc.at(s1 - 1, z, tid), n, nm);
+          cur.mag[L * z + tid] = n;
+          cur.meta[L * z + tid] = nm;
+        }
+      }
+      __syncthreads();
     }
     if (multi) {
       const int wpc = (c.n_full + 31) >> 5;
@@ -412,6 +480,62 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
   }
 }
 
+// Backward of the skipped rows' own columns at iteration t, kOwnGroup rows at a time: gp of an
+// own column holds this iteration's loss gradient alone, and is cleared for the next one.  Returns
+// the buffer of sums to use next.  (Out of line: inlined, its registers made the rows spill.)
+__device__ __noinline__ int own_columns_bwd(const LearnedArgs& a, float* gp, Tape cur, int live, int t,
+                                            const float2* w, float* red, int buf) {
+  const cbd::DevCode& c = a.code;
+  const int z = c.z, nt = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  constexpr int RW = 2 * kMaxLevelEdges;
+  const bool active = tid < z;
+  for (int L0 = live; L0 < c.rows_n; L0 += kOwnGroup) {
+    float v[2 * kOwnGroup];
+    float2 n[kOwnGroup];
+    uint32_t nm[kOwnGroup];
+#pragma unroll
+    for (int j = 0; j < kOwnGroup; j++) {
+      n[j] = make_float2(0.f, 0.f);
+      nm[j] = 0;
+      if (active && L0 + j < c.rows_n) {
+        n[j] = cur.mag[(L0 + j) * z + tid];
+        nm[j] = cur.meta[(L0 + j) * z + tid];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kOwnGroup; j++) {
+      v[2 * j] = v[2 * j + 1] = 0.f;
+      if (active && L0 + j < c.rows_n) {
+        const float2 ab = w[c.layer_start[L0 + j + 1] - 1];
+        float* own = gp + (c.cols_k + L0 + j) * z + tid;
+        const float g = *own, m = n[j].y;
+        *own = 0.f;
+        const float ga = __fmaf_rn(ab.x, m, -ab.y) > 0.f ? ((nm[j] & 1u) ? -g : g) : 0.f;
+        const float gm = ga * ab.x;
+        v[2 * j] = ga * m;
+        v[2 * j + 1] = ga;
+        // (two rows may meet on a variable)
+        atomicAdd(reinterpret_cast<float*>(reinterpret_cast<char*>(gp) + __float_as_int(n[j].x)),
+                  (nm[j] & 2u) ? -gm : gm);
+      }
+    }
+    put_warp_sums(v, red + ((size_t)buf * nw + warp) * RW, lane);
+    __syncthreads();
+    for (int i = tid; i < 2 * kOwnGroup; i += nt) {
+      const int L = L0 + (i >> 1);
+      if (L < c.rows_n) {
+        const float* rd = red + (size_t)buf * nw * RW + i;
+        float sum = 0.f;
+        for (int k = 0; k < nw; k++) sum += rd[k * RW];
+        const size_t wi = (size_t)t * c.n_entries + c.layer_start[L + 1] - 1;
+        atomicAdd((i & 1) ? &a.g_beta[wi] : &a.g_alpha[wi], (i & 1) ? -sum : sum);
+      }
+    }
+    buf ^= 1;
+  }
+  return buf;
+}
+
 template <bool SHARED, int S>
 __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_constant__ LearnedArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -429,6 +553,8 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
   const int wpc = (c.n_full + 31) >> 5;
   const bool multi = a.multi_loss && a.P;
   const bool active = tid < z;
+  const int live = SHARED ? *a.live : c.rows_n, run = live < c.rows_n ? c.rows_run : c.rows_n;
+  const bool own_loss = live < c.rows_n && a.loss_bits > (c.cols_k + live) * z;  // on a skipped row's column
   const float scale = 1.f / ((float)a.loss_bits * (float)a.n_frames);
   for (int v = tid; v < c.n_full; v += nt) gp[v] = 0.f;
   __syncthreads();
@@ -465,11 +591,15 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
     float2 n = make_float2(0.f, 0.f);
     uint32_t nm = 0;
     if (active) {
-      const int i = c.layer_order[c.rows_n - 1] * z + tid;
+      const int i = c.layer_order[run - 1] * z + tid;
       n = cur.mag[i];
       nm = cur.meta[i];
     }
-    for (int q = c.rows_n - 1; q >= 0;) {
+    // the skipped rows, the last of the forward pass
+    if constexpr (SHARED) {
+      if (own_loss && (multi || t == a.T - 1)) buf = own_columns_bwd(a, gp, cur, live, t, wbuf, red, buf);
+    }
+    for (int q = run - 1; q >= 0;) {
       // the rows of a level, then a barrier, then the level's sums into the gradients
       int at = 0, qe = q;
       do {
@@ -484,7 +614,7 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
         }
         float* rd = red + ((size_t)buf * nw + warp) * RW + 2 * at;
 #define CB_ROW(DD)                                                                                                 \
-  learned_row_bwd<DD, SHARED, S>(a, gp, gc + (size_t)s0 * S, n, nm, t, s0, tid, z, active, t == a.T - 1, w, rd, lane);
+  learned_row_bwd<DD, SHARED, S>(a, gp, gc + (size_t)s0 * S, n, nm, t, s0, tid, z, active && L < live, t == a.T - 1, w, rd, lane);
         CB_LEARNED_DEGREES(CB_ROW)
 #undef CB_ROW
         n = nn;
@@ -543,6 +673,10 @@ __global__ void adam_kernel(float* w, const float* g, float* m, float* v, int64_
 }  // namespace
 
 cudaError_t launch_learned(const LearnedArgs& a, bool forward, cudaStream_t s) {
+  if (forward && a.shared) {
+    learned_live_kernel<<<1, 256, 0, s>>>(a);
+    if (cudaError_t e = cudaGetLastError()) return e;
+  }
   const int threads = ((a.code.z + 31) / 32) * 32;
   void* k;
   if (forward) {
