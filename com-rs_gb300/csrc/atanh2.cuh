@@ -72,6 +72,19 @@ inline double from_bits(uint64_t b) {
 inline double tab(int j, int k) { return LOGTAB[j][k]; }
 #endif
 
+// the double of an integer 0 <= e < 2^20 on the integer pipes (the conversion runs on the
+// FP64 pipe, which bounds the caller)
+AT2_HD double small_int(int e) {
+  if (e == 0) return 0.0;
+#if defined(__CUDA_ARCH__)
+  const int top = 31 - __clz(e);
+#else
+  const int top = 31 - __builtin_clz((unsigned)e);
+#endif
+  const uint32_t hi = ((uint32_t)(1022 + top) << 20) + ((uint32_t)e << (20 - top));  // the leading one adds the last 1
+  return from_bits((uint64_t)hi << 32);
+}
+
 // 2 atanh(clamp(p, -bound, bound)) (see the header comment for the domain)
 AT2_HD double twice_atanh(double p, double bound) {
   const uint64_t sign = bits(p) & 0x8000000000000000ull;
@@ -106,7 +119,7 @@ AT2_HD double twice_atanh(double p, double bound) {
   double qp = LOGTAB_Q[LOGTAB_Q_TERMS - 1];
   for (int k = LOGTAB_Q_TERMS - 2; k >= 0; k--) qp = fma_rn(qp, r, LOGTAB_Q[k]);
   const double r2 = mul(r, r);
-  const double ed = (double)e;
+  const double ed = small_int(e);
   const double hi = fma_rn(ed, LOGTAB_LN2_HI, lhi);  // exact
   double lo = fma_rn(ed, LOGTAB_LN2_LO, llo);
   lo = add(lo, delta);
@@ -117,7 +130,8 @@ AT2_HD double twice_atanh(double p, double bound) {
   double res = add(S, add(err, lo));
   // a < 2^-27: 2 atanh(a) = 2a (1 + a^2/3 + ...) rounds to 2a, which the sum above misses
   // by up to an ulp when ul is as large as the result
-  if (ab < 0x3e40000000000000ull) res = add(a, a);
+  // (2a from its bits: the exponent one more, a subnormal shifted)
+  if (ab < 0x3e40000000000000ull) res = from_bits((ab >> 52) ? ab + 0x0010000000000000ull : ab << 1);
   return from_bits(bits(res) | sign);
 }
 
