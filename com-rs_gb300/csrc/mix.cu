@@ -2,10 +2,8 @@
 // modulations decoded by one persistent kernel, each with its own early exit.
 //
 // The batch's codewords are sorted by lifting size into classes.  The kernel walks the
-// classes in order; for class k every CTA, one per SM, splits its threads into `slots` groups of
-// `slot_threads` threads (a multiple of 32, synchronised by their own named barrier).  One
-// CTA of 768 threads instead of two of 384: Z = 208 then has three slots of seven warps on an
-// SM and not two, Z = 128 five of four warps and not four (@MIX@).
+// classes in order; for class k every CTA splits its 384 threads into `slots` groups of
+// `slot_threads` threads (a multiple of 32, synchronised by their own named barrier).
 // Each slot pulls one codeword after another from the class's atomic queue (work
 // stealing), decodes it with the layered min-sum of decode.cu (the same row updates,
 // the same syndrome test, so every result equals the single-code path bit for bit) and
@@ -20,11 +18,7 @@
 namespace cbk {
 namespace {
 
-// a slot of one warp needs no barrier of the CTA's sixteen
-__device__ __forceinline__ void slot_sync(int bar, int n) {
-  if (n == 32) __syncwarp();
-  else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory");
-}
+__device__ __forceinline__ void slot_sync(int bar, int n) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory"); }
 
 // OR of `bad` over the slot's threads (flag starts at 0 and is left at 0)
 __device__ __forceinline__ bool slot_any(int bad, int* flag, int bar, int n, int lt) {
@@ -180,13 +174,13 @@ __device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned 
   }
 }
 
-__global__ void __launch_bounds__(kMixThreads, 1) mix_decode_kernel(const __grid_constant__ MixDecodeArgs a) {
+__global__ void __launch_bounds__(384, 2) mix_decode_kernel(const __grid_constant__ MixDecodeArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ long long s_item[kMixMaxSlots];
-  __shared__ int s_flag[kMixMaxSlots];
-  __shared__ unsigned int s_err[kMixMaxSlots];
+  __shared__ long long s_item[16];
+  __shared__ int s_flag[16];
+  __shared__ unsigned int s_err[16];
   const int tid = threadIdx.x;
-  if (tid < kMixMaxSlots) {
+  if (tid < 16) {
     s_flag[tid] = 0;
     s_err[tid] = 0;
   }
@@ -227,7 +221,7 @@ int mix_decode_grid(size_t smem, int device) {
   void* k = (void*)mix_decode_kernel;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
   int per_sm = 0, sms = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kMixThreads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 384, smem);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   return per_sm * sms;
 }
@@ -237,7 +231,7 @@ cudaError_t launch_mix_decode(const MixDecodeArgs& a, int grid, size_t smem, cud
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void* args[] = {(void*)&a};
-  return cudaLaunchKernel(k, dim3(grid), dim3(kMixThreads), args, smem, s);
+  return cudaLaunchKernel(k, dim3(grid), dim3(384), args, smem, s);
 }
 
 }  // namespace cbk
