@@ -18,8 +18,7 @@
 
 namespace {
 thread_local std::string g_mix_error;
-constexpr size_t kSlotSmemBudget = 113 * 1024;  // two 384-thread CTAs per SM
-constexpr int kCtaThreads = 384;
+constexpr size_t kSlotSmemBudget = 224 * 1024;  // one CTA per SM
 }  // namespace
 
 struct cb_mix {
@@ -75,11 +74,12 @@ void layout(cbk::MixClass& k, int rho) {
   k.slot_threads = std::max(32, ((rows + 31) / 32) * 32);
   k.rows_per_thread = rho;
   k.smem_per_slot = (int32_t)cbk::mix_slot_smem_bytes(k.z);
-  int by_threads = kCtaThreads / k.slot_threads;
+  int by_threads = cbk::kMixThreads / k.slot_threads;
   int by_smem = (int)(kSlotSmemBudget / (size_t)k.smem_per_slot);
-  k.slots = std::min({by_threads, by_smem, 15});
+  k.slots = std::min({by_threads, by_smem, k.slot_threads == 32 ? cbk::kMixMaxSlots : 15});
   k.state_per_slot = (int32_t)((size_t)cbh::kMaxLayers * k.z * 12);
   k.max_ncol = 68;
+  k.straight = rho == 1 && k.slot_threads >= 128 ? 1 : 0;
 }
 
 // sizes that depend on the class layouts: shared memory, state, grid
@@ -255,9 +255,14 @@ cb_status cb_mix_create(const cb_mix_item* items, int64_t n, uint64_t seed, uint
     it.b_ebn0 = b * std::pow(10.0, d.ebn0_db / 10.0);
     it.index = (int32_t)i;
   }
-  // classes by lifting size, largest first
+  // classes by lifting size, largest first; in a class the codewords with the most entries to
+  // update first, so that the last ones to be taken are short
+  std::vector<int> work(m->codes.size());
+  for (size_t i = 0; i < work.size(); i++)
+    work[i] = m->codes[i].layer_start[cbk::decoder_rows(m->codes[i], (double)m->alpha)];
   std::stable_sort(its.begin(), its.end(), [&](const cbk::MixItem& a, const cbk::MixItem& b) {
-    return m->codes[a.code].z > m->codes[b.code].z;
+    const int za = m->codes[a.code].z, zb = m->codes[b.code].z;
+    return za != zb ? za > zb : work[a.code] > work[b.code];
   });
   int64_t llr = 0, info = 0;
   for (int64_t i = 0; i < n; i++) {

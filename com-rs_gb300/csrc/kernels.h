@@ -134,11 +134,14 @@ struct GenMixArgs {
 };
 cudaError_t launch_gen_mix(const GenMixArgs& a, size_t smem, cudaStream_t stream);
 
-// a lifting-size class of a mixed batch and its slot layout in a 384-thread CTA
+constexpr int kMixThreads = 768;   // of a decoder CTA, one per SM
+constexpr int kMixMaxSlots = 24;   // of one warp; at most 15 of more (named barriers 1 to 15)
+// a lifting-size class of a mixed batch and its slot layout in a CTA
 struct MixClass {
   int32_t z, slot_threads, slots, rows_per_thread;
   int64_t first, count;  // its items in the sorted batch
-  int32_t smem_per_slot, state_per_slot, max_ncol, reserved;
+  int32_t smem_per_slot, state_per_slot, max_ncol;
+  int32_t straight;  // 1: the rows with the base graph at compile time (one row per thread)
 };
 struct MixDecodeArgs {
   const cbd::DevCode* codes;

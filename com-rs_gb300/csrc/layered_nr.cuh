@@ -175,8 +175,9 @@ struct NrTuning {
 // column's offset is an immediate of the shared-memory access.  (A comparison of r with
 // Z - shift selecting between two immediates issues more instructions: 17.6 against
 // 16.7 ms per 8192 C2 codewords.)
-template <int BG, class K, int T>
-__device__ __forceinline__ int edge_offset(const NrArgs& a, int r, int r4, int z4) {
+// (A: the launch parameters, or anything with the table `eaddr` of the runtime lifting.)
+template <int BG, class K, int T, class A>
+__device__ __forceinline__ int edge_offset(const A& a, int r, int r4, int z4) {
   if constexpr (K::fixed) {
     constexpr int sh = K::shift[T], c = Graph<BG>::col[T];
     const uint32_t u = (uint32_t)r4 + (uint32_t)(4 * sh);
@@ -190,8 +191,8 @@ __device__ __forceinline__ int edge_offset(const NrArgs& a, int r, int r4, int z
 }
 
 // the edge offsets of a row, entries S0 + I .. S0 + D - 1 (a compile-time loop)
-template <int BG, class K, int S0, int I, int D>
-__device__ __forceinline__ void row_offsets(int (&off)[D], const NrArgs& a, int r, int r4, int z4) {
+template <int BG, class K, int S0, int I, int D, class A>
+__device__ __forceinline__ void row_offsets(int (&off)[D], const A& a, int r, int r4, int z4) {
   if constexpr (I < D) {
     off[I] = edge_offset<BG, K, S0 + I>(a, r, r4, z4);
     row_offsets<BG, K, S0, I + 1, D>(off, a, r, r4, z4);
@@ -208,8 +209,8 @@ __device__ __forceinline__ void st_f(unsigned char* post, int off, float v) {
 // One lifted row of base row L (degree D, entries S0 ..): old state (a1, a2, mt) -> new
 // state (n1, n2, nm), posteriors updated in place.  The operations of row_update_lean
 // (decode_common.cuh), with the addresses from edge_offset.
-template <int BG, class K, int S0, int D, int RULE>
-__device__ __forceinline__ void nr_row(unsigned char* post, const NrArgs& a, int r, int r4, int z4, float a1,
+template <int BG, class K, int S0, int D, int RULE, class A>
+__device__ __forceinline__ void nr_row(unsigned char* post, const A& a, int r, int r4, int z4, float a1,
                                        float a2, uint32_t mt, float alpha, float& n1, float& n2, uint32_t& nm) {
   int off[D];
   float x[D];

@@ -2,8 +2,11 @@
 // modulations decoded by one persistent kernel, each with its own early exit.
 //
 // The batch's codewords are sorted by lifting size into classes.  The kernel walks the
-// classes in order; for class k every CTA splits its 384 threads into `slots` groups of
-// `slot_threads` threads (a multiple of 32, synchronised by their own named barrier).
+// classes in order; for class k every CTA, one per SM, splits its threads into `slots` groups of
+// `slot_threads` threads (a multiple of 32, synchronised by their own named barrier).  One
+// CTA of 768 threads instead of two of 384: Z = 208 then has three slots of seven warps on an
+// SM and not two, Z = 128 five of four warps and not four (the decode phase of 16384
+// uneven codewords 9.0 -> 8.6 ms).
 // Each slot pulls one codeword after another from the class's atomic queue (work
 // stealing), decodes it with the layered min-sum of decode.cu (the same row updates,
 // the same syndrome test, so every result equals the single-code path bit for bit) and
@@ -14,11 +17,16 @@
 
 #include "decode_common.cuh"
 #include "kernels.h"
+#include "layered_nr.cuh"
 
 namespace cbk {
 namespace {
 
-__device__ __forceinline__ void slot_sync(int bar, int n) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory"); }
+// a slot of one warp needs no barrier of the CTA's sixteen
+__device__ __forceinline__ void slot_sync(int bar, int n) {
+  if (n == 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory");
+}
 
 // OR of `bad` over the slot's threads (flag starts at 0 and is left at 0)
 __device__ __forceinline__ bool slot_any(int bad, int* flag, int bar, int n, int lt) {
@@ -72,7 +80,40 @@ __device__ bool slot_check_fails(const float* post, uint32_t* hd, const uint32_t
   return slot_any(bad, flag, bar, nt, lt);
 }
 
-// Decode one codeword of the batch in a slot; RHO rows per thread.
+// The rows of one iteration with the base graph's structure at compile time
+// (layered_nr.cuh), the edge addresses from the slot's table.  Bound by issue: the degree and
+// the entries' bounds are no longer read and branched on per row.  Used for slots of at
+// least 128 threads; 16384 uneven codewords, generator and decoder: 9.32 ms, 9.99 with no
+// slot on it, 9.41 from 256 threads, 9.52 from 64 and 9.70 with all slots on it.
+struct MixTable {
+  const uint2* eaddr;  // {4 shift, 4 column Z} per entry
+};
+template <int BG, int Q>
+__device__ __forceinline__ void mix_rows(unsigned char* post, const MixTable& tab, const StateSlot<float>& st, int lt,
+                                         int z, bool first, float alpha, int live, int bar, int nt) {
+  using G = cbn::Graph<BG>;
+  if constexpr (Q < G::rows) {
+    if constexpr (Q >= 4) {
+      if constexpr (G::level_end[Q - 1] != 0) {
+        if (live <= cbn::rest_min<BG>(Q)) return;
+      }
+    }
+    constexpr int L = G::order[Q], S0 = G::start[L], D = G::start[L + 1] - S0;
+    if (lt < z) {
+      int r = lt;
+      asm volatile("" : "+r"(r));  // (addresses formed where they are used, see nr_iteration)
+      float a1 = 0.f, a2 = 0.f, n1, n2;
+      uint32_t mt = 0u, nm;
+      if (!first) st.load(L * z + r, a1, a2, mt);
+      cbn::nr_row<BG, cbn::RuntimeLifting, S0, D, 1>(post, tab, r, 4 * r, 4 * z, a1, a2, mt, alpha, n1, n2, nm);
+      st.store(L * z + r, n1, n2, nm);
+    }
+    if constexpr (G::level_end[Q] != 0) slot_sync(bar, nt);
+    mix_rows<BG, Q + 1>(post, tab, st, lt, z, first, alpha, live, bar, nt);
+  }
+}
+
+// Decode one codeword of the batch in a slot; RHO rows per thread (0: one, by mix_rows).
 template <int RHO>
 __device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned char* sm, int ncol_max,
                             const StateSlot<float>& st, int lt, int nt, int bar, int* flag, unsigned int* err) {
@@ -88,8 +129,9 @@ __device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned 
   uint8_t* s_end = s_order + cbh::kMaxLayers;
   const int ncol = c.n_full / z;
   for (int i = lt; i < c.n_entries; i += nt) {
-    s_ent[i] = c.entry[i];
-    s_addr[i] = c.eaddr[i];
+    const uint32_t en = c.entry[i];
+    s_ent[i] = en;
+    s_addr[i] = RHO ? c.eaddr[i] : make_uint2(4u * (en & 0xffffu), 4u * (en >> 16) * (uint32_t)z);
   }
   for (int i = lt; i <= c.rows_n; i += nt) s_lstart[i] = c.layer_start[i];
   for (int i = lt; i < c.rows_n; i += nt) {
@@ -113,7 +155,12 @@ __device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned 
     for (int iter = 1; iter <= a.max_it; iter++) {
       // the base rows by levels, as decode.cu runs them; each row's state is loaded where
       // it is used (loaded one row ahead: 17.56 against 17.40 ms per decode phase)
-      for (int k = 0; k < rows_run; k++) {
+      if constexpr (RHO == 0) {
+        unsigned char* pb = reinterpret_cast<unsigned char*>(post);
+        if (c.bg == 1) mix_rows<1, 0>(pb, MixTable{s_addr}, st, lt, z, iter == 1, a.alpha, rows_live, bar, nt);
+        else mix_rows<2, 0>(pb, MixTable{s_addr}, st, lt, z, iter == 1, a.alpha, rows_live, bar, nt);
+      }
+      for (int k = 0; RHO && k < rows_run; k++) {
         const int L = s_order[k];
         const int s0 = s_lstart[L], d = s_lstart[L + 1] - s0;
 #pragma unroll
@@ -174,13 +221,13 @@ __device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned 
   }
 }
 
-__global__ void __launch_bounds__(384, 2) mix_decode_kernel(const __grid_constant__ MixDecodeArgs a) {
+__global__ void __launch_bounds__(kMixThreads, 1) mix_decode_kernel(const __grid_constant__ MixDecodeArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ long long s_item[16];
-  __shared__ int s_flag[16];
-  __shared__ unsigned int s_err[16];
+  __shared__ long long s_item[kMixMaxSlots];
+  __shared__ int s_flag[kMixMaxSlots];
+  __shared__ unsigned int s_err[kMixMaxSlots];
   const int tid = threadIdx.x;
-  if (tid < 16) {
+  if (tid < kMixMaxSlots) {
     s_flag[tid] = 0;
     s_err[tid] = 0;
   }
@@ -188,7 +235,12 @@ __global__ void __launch_bounds__(384, 2) mix_decode_kernel(const __grid_constan
   for (int k = 0; k < a.n_classes; k++) {
     const MixClass cls = a.classes[k];
     const int slot = tid / cls.slot_threads;
-    if (slot < cls.slots) {
+    // A CTA opens at most twice its share of the class in slots: with all of them open, the
+    // first CTAs take a small class whole and decode it on a few SMs (300 codewords,
+    // generator and decoder: 0.97 against 0.81 ms).  One share leaves slots idle in the later
+    // classes (2000 codewords 1.83 against 1.71 ms; three shares 1.76).
+    const int share = (int)min((cls.count + gridDim.x - 1) / (long long)gridDim.x, (long long)kMixMaxSlots);
+    if (slot < min(cls.slots, 2 * share)) {
       const int lt = tid - slot * cls.slot_threads, nt = cls.slot_threads, bar = slot + 1;
       unsigned char* sm = smem + (size_t)slot * cls.smem_per_slot;
       const StateSlot<float> st(a.state + (size_t)blockIdx.x * a.state_per_cta + (size_t)slot * cls.state_per_slot,
@@ -200,7 +252,8 @@ __global__ void __launch_bounds__(384, 2) mix_decode_kernel(const __grid_constan
         slot_sync(bar, nt);
         if (i >= cls.count) break;
         const MixItem it = a.items[cls.first + i];
-        if (cls.rows_per_thread == 1) decode_item<1>(a, it, sm, cls.max_ncol, st, lt, nt, bar, &s_flag[slot], &s_err[slot]);
+        if (cls.straight) decode_item<0>(a, it, sm, cls.max_ncol, st, lt, nt, bar, &s_flag[slot], &s_err[slot]);
+        else if (cls.rows_per_thread == 1) decode_item<1>(a, it, sm, cls.max_ncol, st, lt, nt, bar, &s_flag[slot], &s_err[slot]);
         else decode_item<2>(a, it, sm, cls.max_ncol, st, lt, nt, bar, &s_flag[slot], &s_err[slot]);
       }
     }
@@ -221,7 +274,7 @@ int mix_decode_grid(size_t smem, int device) {
   void* k = (void*)mix_decode_kernel;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
   int per_sm = 0, sms = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 384, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kMixThreads, smem);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   return per_sm * sms;
 }
@@ -231,7 +284,7 @@ cudaError_t launch_mix_decode(const MixDecodeArgs& a, int grid, size_t smem, cud
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void* args[] = {(void*)&a};
-  return cudaLaunchKernel(k, dim3(grid), dim3(384), args, smem, s);
+  return cudaLaunchKernel(k, dim3(grid), dim3(kMixThreads), args, smem, s);
 }
 
 }  // namespace cbk
