@@ -31,6 +31,7 @@
 
 #include "decode_common.cuh"
 #include "kernels.h"
+#include "layered_nr.cuh"
 
 namespace cbk {
 namespace {
@@ -92,6 +93,72 @@ __device__ __forceinline__ void decode_layers(const cbd::DevCode& c, T* post, co
     }
     if (c.level_end[q]) __syncthreads();
   }
+}
+
+// The positions of a row's variables, the columns at compile time
+template <int D>
+struct OffsetsAt {
+  int off[D];
+  __device__ __forceinline__ int operator()(int e) const { return off[e]; }
+};
+template <int BG, int S0, int I, int D>
+__device__ __forceinline__ void row_positions(int (&off)[D], const cbd::DevCode& c, int r, int z) {
+  if constexpr (I < D) {
+    constexpr int col = cbn::Graph<BG>::col[S0 + I];
+    const unsigned v = c.entry[S0 + I] - ((unsigned)col << 16) + (unsigned)r;
+    off[I] = col * z + (int)min(v, v - (unsigned)z);
+    row_positions<BG, S0, I + 1, D>(off, c, r, z);
+  }
+}
+
+// One layered iteration of the f64 decoder with the base graph at compile time
+// (layered_nr.cuh has its schedule), for grids that leave an SM few codewords: a row then
+// waits for a chain of loads (its index, its entries' bounds, the entries, its state), of
+// which the posteriors alone are left.  The state is loaded a row ahead (152 codewords of
+// BG2 Z = 52, generator and decoder: 0.486 ms by decode_layers, 0.448 with the state loaded
+// at its use, 0.42 to 0.44 ahead; 96 words of BG1 Z = 144 from host memory 0.46 -> 0.42).  A
+// full device gains nothing at BG2 Z = 52 and loses at BG1 Z = 64 (2000 codewords 3.57 ->
+// 4.18 ms), so it keeps decode_layers.
+template <int BG, int RULE, int Q>
+__device__ __forceinline__ void decode_rows(const cbd::DevCode& c, double* post, const StateSlot<double>& st,
+                                            bool first, int r, int z, bool active, const ScaleF64& scale, double a1,
+                                            double a2, uint32_t mt) {
+  using G = cbn::Graph<BG>;
+  if constexpr (Q < G::rows) {
+    if constexpr (Q >= 4) {
+      if constexpr (G::level_end[Q - 1] != 0) {
+        if (c.rows_live <= cbn::rest_min<BG>(Q)) return;
+      }
+    }
+    constexpr int L = G::order[Q], S0 = G::start[L], D = G::start[L + 1] - S0;
+    double b1 = 0.0, b2 = 0.0;
+    uint32_t bt = 0u;
+    if (active) {
+      int rr = r, zz = z;
+      // addresses formed where they are used: kept over the iterations, the rows' state
+      // addresses alone spill 420 bytes
+      asm volatile("" : "+r"(rr), "+r"(zz));
+      if constexpr (Q + 1 < G::rows) {
+        if (!first) st.load(G::order[Q + 1] * zz + rr, b1, b2, bt);
+      }
+      double n1, n2;
+      uint32_t nm;
+      OffsetsAt<D> at;
+      row_positions<BG, S0, 0, D>(at.off, c, rr, zz);
+      row_update<D, RULE, false>(post, at, a1, a2, mt, scale, n1, n2, nm);
+      st.store(L * zz + rr, n1, n2, nm);
+    }
+    if constexpr (G::level_end[Q] != 0) __syncthreads();
+    decode_rows<BG, RULE, Q + 1>(c, post, st, first, r, z, active, scale, b1, b2, bt);
+  }
+}
+template <int BG, int RULE>
+__device__ __forceinline__ void decode_rows(const cbd::DevCode& c, double* post, const StateSlot<double>& st,
+                                            bool first, int r, int z, bool active, const ScaleF64& scale) {
+  double a1 = 0.0, a2 = 0.0;
+  uint32_t mt = 0u;
+  if (active && !first) st.load(cbn::Graph<BG>::order[0] * z + r, a1, a2, mt);
+  decode_rows<BG, RULE, 0>(c, post, st, first, r, z, active, scale, a1, a2, mt);
 }
 
 template <typename T, int LW, int MAXD, bool FULL>
@@ -200,7 +267,13 @@ __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float*
         // the rows of one iteration, the rule a template parameter (one branch around the
         // whole iteration, none in the rows)
         const LearnedRowW lw{w_ap, w_bp, w_ac, w_bc, 0, w_stride, w_roff};  // (of this thread's row)
-        if (LEARNED || rule == cbd::RULE_NMS)
+        if constexpr (sizeof(T) == 8 && !FULL) {
+          constexpr int BG = MAXD == 19 ? 1 : 2;
+          if (rule == cbd::RULE_NMS)
+            decode_rows<BG, cbd::RULE_NMS>(c, post, st, iter == 1, tid, z, active, scale);
+          else
+            decode_rows<BG, cbd::RULE_OMS>(c, post, st, iter == 1, tid, z, active, scale);
+        } else if (LEARNED || rule == cbd::RULE_NMS)
           decode_layers<T, LW, cbd::RULE_NMS, MAXD, FULL>(c, post, st, lw, iter, tid, z, active, alpha, scale);
         else
           decode_layers<T, LW, cbd::RULE_OMS, MAXD, FULL>(c, post, st, lw, iter, tid, z, active, alpha, scale);
@@ -280,14 +353,15 @@ __global__ void __launch_bounds__(384, 2) layered_learned_param_kernel(const __g
   decode_body<float, kWeightsParam, 19, true>(a.d, a.alpha, a.beta);
 }
 
-// The plain decoder.  f64 has four builds: codes without rows of more than 10 edges (base
-// graph 2: 126 registers instead of 148), and, when every SM has its CTAs, the scaling's
-// products on the integer pipes and the next row's state loaded ahead.  Those take the FP64
-// pipe's time, not the latency of a row, of which a codeword alone on an SM is made: with them 96
-// codewords of BG1 Z = 144 take 1-3 % longer, 4096 of BG2 Z = 52 8 % less.
-void* plain_kernel(int precision, int max_degree, bool full) {
+// The plain decoder.  f64 has four builds: per base graph (2, with rows of at most 10 edges,
+// takes fewer registers), and by whether every SM has its CTAs.  If so, the FP64 pipe bounds
+// the rows: the scaling's products on the integer pipes, the next row's state loaded ahead
+// (4096 codewords of BG2 Z = 52: 8 % less time).  If not, the latency of a row does:
+// decode_rows, and the scaling as two multiplications (on the integer pipes 96 codewords of
+// BG1 Z = 144 take 1-3 % longer).
+void* plain_kernel(int precision, int bg, bool full) {
   if (precision == 1) return (void*)layered_kernel<float, kPlain, 19, true>;
-  if (max_degree <= 10)
+  if (bg == 2)
     return full ? (void*)layered_kernel<double, kPlain, 10, true> : (void*)layered_kernel<double, kPlain, 10, false>;
   return full ? (void*)layered_kernel<double, kPlain, 19, true> : (void*)layered_kernel<double, kPlain, 19, false>;
 }
@@ -297,7 +371,7 @@ void* kernel_for(const DecodeArgs<T>& a, int grid) {
   if constexpr (sizeof(T) == 4) {
     if (a.l_alpha) return a.l_smem ? (void*)layered_kernel<T, kWeightsShared, 19, true> : (void*)layered_kernel<T, kWeightsGlobal, 19, true>;
   }
-  return plain_kernel(sizeof(T) == 8 ? 0 : 1, a.code.max_degree, grid >= a.full_grid);
+  return plain_kernel(sizeof(T) == 8 ? 0 : 1, a.code.bg, grid >= a.full_grid);
 }
 
 int block_threads(int z) { return ((z + 31) / 32) * 32; }
@@ -315,7 +389,7 @@ size_t decode_state_bytes_per_slot(const cbd::DevCode& c, int precision) {
 }
 
 int decode_grid_size(const cbd::DevCode& c, int precision, int device) {
-  void* k = plain_kernel(precision, c.max_degree, true);
+  void* k = plain_kernel(precision, c.bg, true);
   size_t smem = smem_bytes(c, precision);
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0, sms = 0;

@@ -12,6 +12,18 @@
 namespace cbk {
 namespace {
 
+// Position in post of edge e's variable for lifted row r, from the packed entries
+struct EntryAt {
+  const uint32_t* ent;
+  int r, z;
+  __device__ __forceinline__ int operator()(int e) const {
+    const uint32_t en = ent[e];
+    // (r + shift) mod Z with one unsigned min: r + shift < 2Z
+    const unsigned c = (unsigned)r + (en & 0xffffu);
+    return (int)(en >> 16) * z + (int)min(c, c - (unsigned)z);
+  }
+};
+
 // One lifted row of a layer in f64: thread r, degree D known at compile time.
 // old state (a1, a2, mt) -> new state (n1, n2, nm); post updated in place.
 // RULE (cbd::RULE_NMS or RULE_OMS) is a template parameter: with the rule read at run time
@@ -22,20 +34,16 @@ namespace {
 // doubles is that of their bit patterns, and with FULL the normalised rule's products are formed by
 // scaled() (4096 frames of BG2 Z = 52 at 9.7 iterations: 3.00 -> 2.80 ms; the pipe 71 % busy,
 // where a kernel of additions alone reaches 84 %).
-template <int D, int RULE, bool FULL>
-__device__ __forceinline__ void row_update(double* __restrict__ post, const uint32_t* __restrict__ ent, int r, int z,
-                                           double a1, double a2, uint32_t mt, const ScaleF64& scale, double& n1,
-                                           double& n2, uint32_t& nm) {
+// `at` gives the position in post of edge e's variable.
+template <int D, int RULE, bool FULL, typename At>
+__device__ __forceinline__ void row_update(double* __restrict__ post, const At& at, double a1, double a2, uint32_t mt,
+                                           const ScaleF64& scale, double& n1, double& n2, uint32_t& nm) {
   int off[D];
   double x[D];
   const int old_i1 = (int)(mt & 31u);
 #pragma unroll
   for (int e = 0; e < D; e++) {
-    const uint32_t en = ent[e];
-    // (r + shift) mod Z with one unsigned min: r + shift < 2Z
-    unsigned c = (unsigned)r + (en & 0xffffu);
-    unsigned cm = c - (unsigned)z;
-    off[e] = (int)(en >> 16) * z + (int)min(c, cm);
+    off[e] = at(e);
     // the old message as bits: the magnitude (never negative) with the old sign ORed
     // in, so that one subtraction is the FP64 work (p - (-m) is p + m, bit for bit)
     const long long mb = __double_as_longlong(e == old_i1 ? a2 : a1);
@@ -267,16 +275,16 @@ __device__ __forceinline__ void row_dispatch(int d, double* post, const uint32_t
                                              double a2, uint32_t mt, const ScaleF64& scale, double& n1, double& n2,
                                              uint32_t& nm) {
   switch (d) {
-    case 3: row_update<3, RULE, FULL>(post, ent, r, z, a1, a2, mt, scale, n1, n2, nm); break;
-    case 4: row_update<4, RULE, FULL>(post, ent, r, z, a1, a2, mt, scale, n1, n2, nm); break;
-    case 5: row_update<5, RULE, FULL>(post, ent, r, z, a1, a2, mt, scale, n1, n2, nm); break;
-    case 6: row_update<6, RULE, FULL>(post, ent, r, z, a1, a2, mt, scale, n1, n2, nm); break;
-    case 7: row_update<7, RULE, FULL>(post, ent, r, z, a1, a2, mt, scale, n1, n2, nm); break;
-    case 8: row_update<8, RULE, FULL>(post, ent, r, z, a1, a2, mt, scale, n1, n2, nm); break;
-    case 9: row_update<9, RULE, FULL>(post, ent, r, z, a1, a2, mt, scale, n1, n2, nm); break;
-    case 10: row_update<10, RULE, FULL>(post, ent, r, z, a1, a2, mt, scale, n1, n2, nm); break;
+    case 3: row_update<3, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 4: row_update<4, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 5: row_update<5, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 6: row_update<6, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 7: row_update<7, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 8: row_update<8, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 9: row_update<9, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 10: row_update<10, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
     default:
-      if constexpr (MAXD > 10) row_update<19, RULE, FULL>(post, ent, r, z, a1, a2, mt, scale, n1, n2, nm);
+      if constexpr (MAXD > 10) row_update<19, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm);
       break;
   }
 }
