@@ -423,7 +423,10 @@ cudaError_t ensure_map(cb_code* c) {
   const cbh::NrCode& h = c->host;
   int32_t* p = nullptr;
   cudaError_t e = cudaMalloc(&p, sizeof(int32_t) * h.e);
-  if (e == cudaSuccess) e = cudaMemcpy(p, h.map.data(), sizeof(int32_t) * h.e, cudaMemcpyHostToDevice);
+  // (not on the legacy stream: a caller may be capturing a stream that synchronises with it)
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(p, h.map.data(), sizeof(int32_t) * h.e, cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     cudaFree(p);
     return e;
@@ -437,7 +440,7 @@ cudaError_t ensure_map(cb_code* c) {
 // Only the stream and the rate matching's map are set up: encoding needs no decoder.  The
 // caller's current device stays what it was, and a stream capture of the calling thread
 // goes on undisturbed (the relaxed mode allows the allocations made here).
-cudaError_t encode_device(cb_code* c, const uint8_t* info, int64_t n, uint8_t* out) {
+cudaError_t encode_device(cb_code* c, const uint8_t* info, int64_t n, uint8_t* out, bool* ready) {
   struct Restore {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     int device = -1;
@@ -458,6 +461,7 @@ cudaError_t encode_device(cb_code* c, const uint8_t* info, int64_t n, uint8_t* o
   const int64_t chunk = std::min<int64_t>(n, std::max<int64_t>(1, (int64_t)(((size_t)256 << 20) / per)));
   // the sent bytes first: their rows are 4-byte aligned when E is a multiple of 4
   if (e == cudaSuccess) e = grow(c->d_u8, c->u8_cap, (size_t)chunk * per);
+  *ready = e == cudaSuccess;
   for (int64_t done = 0; done < n && e == cudaSuccess; done += chunk) {
     const int64_t cnt = std::min(chunk, n - done);
     cbk::NrEncodeArgs a;
@@ -687,10 +691,11 @@ cb_status cb_encode(cb_code* c, const uint8_t* info, int64_t n, uint8_t* out) {
       c->encode_on = c->device >= 0 && c->device < count ? 1 : 2;
     }
     if (c->encode_on == 1) {
-      const cudaError_t e = encode_device(c, info, n, out);
+      bool ready = false;
+      const cudaError_t e = encode_device(c, info, n, out, &ready);
       if (e == cudaSuccess) return CB_OK;
-      if (e != cudaErrorMemoryAllocation) return cuda_fail(c, e, "cb_encode");
-      cudaGetLastError();  // no device memory to spare: the host encodes
+      if (ready) return cuda_fail(c, e, "cb_encode");
+      cudaGetLastError();  // no stream or memory to be had on the device: the host encodes
     }
   }
   // the host encoder, over the same construction tables
