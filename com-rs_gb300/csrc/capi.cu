@@ -1336,7 +1336,10 @@ cb_status decode_noalloc_impl(cb_code* c, void* scratch, const T* llr, int64_t n
     return fail(c, CB_ERR_SHAPE,
                 "the check-node state of one CTA (" + std::to_string(slot) + " bytes) exceeds the " +
                     std::to_string(kNoallocScratchBytes >> 20) + " MiB scratch of cb_decode_device_noalloc");
-  if (c->noalloc_grid <= 0)  // the occupancy query once per code object
+  // once per code object: the occupancy query, and the load of the builds that this and
+  // other codes may take, so that no later call maps device memory for one
+  if (c->noalloc_grid <= 0 && !use_nr) CB_CUDA(c, cbk::decode_load(c->precision));
+  if (c->noalloc_grid <= 0)
     c->noalloc_grid = use_nr ? cbk::nr_grid_size(k, c->host, c->device)
                              : cbk::decode_grid_size(c->dev, c->precision, c->device);
   const int occupancy = c->noalloc_grid;
@@ -1362,6 +1365,7 @@ cb_status decode_noalloc_impl(cb_code* c, void* scratch, const T* llr, int64_t n
     return CB_OK;
   }
   cbk::DecodeArgs<T> a;
+  a.full_grid = occupancy;
   a.code = c->dev;
   a.cfg = c->cfg;
   a.llr = llr;

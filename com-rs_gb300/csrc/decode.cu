@@ -116,7 +116,7 @@ __device__ __forceinline__ void row_positions(int (&off)[D], const cbd::DevCode&
 // waits for a chain of loads (its index, its entries' bounds, the entries, its state), of
 // which the posteriors alone are left.  The state is loaded a row ahead (152 codewords of
 // BG2 Z = 52, generator and decoder: 0.486 ms by decode_layers, 0.448 with the state loaded
-// at its use, 0.42 to 0.44 ahead; 96 words of BG1 Z = 144 from host memory 0.46 -> 0.42).  A
+// at its use, 0.42 to 0.44 ahead; 96 words of BG2 Z = 304 from host memory 0.46 -> 0.42).  A
 // full device gains nothing at BG2 Z = 52 and loses at BG1 Z = 64 (2000 codewords 3.57 ->
 // 4.18 ms), so it keeps decode_layers.
 template <int BG, int RULE, int Q>
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(384, 2) layered_learned_param_kernel(const __g
 // the rows: the scaling's products on the integer pipes, the next row's state loaded ahead
 // (4096 codewords of BG2 Z = 52: 8 % less time).  If not, the latency of a row does:
 // decode_rows, and the scaling as two multiplications (on the integer pipes 96 codewords of
-// BG1 Z = 144 take 1-3 % longer).
+// BG2 Z = 304 take 1-3 % longer).
 void* plain_kernel(int precision, int bg, bool full) {
   if (precision == 1) return (void*)layered_kernel<float, kPlain, 19, true>;
   if (bg == 2)
@@ -396,6 +396,13 @@ int decode_grid_size(const cbd::DevCode& c, int precision, int device) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, block_threads(c.z), smem);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   return per_sm * sms;
+}
+
+cudaError_t decode_load(int precision) {
+  cudaFuncAttributes attr;
+  for (int i = 0; i < 4; i++)
+    if (cudaError_t e = cudaFuncGetAttributes(&attr, plain_kernel(precision, 1 + (i & 1), i < 2))) return e;
+  return cudaSuccess;
 }
 
 template <typename T>

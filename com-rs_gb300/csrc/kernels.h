@@ -46,6 +46,9 @@ cudaError_t launch_decode_learned_param(const LearnedParamArgs& a, int grid, cud
 // the number of resident CTAs the persistent decoder launches and the state each needs
 int decode_grid_size(const cbd::DevCode& code, int precision, int device);
 size_t decode_state_bytes_per_slot(const cbd::DevCode& code, int precision);
+// loads every build of the plain decoder (a kernel's first use otherwise maps its code into
+// device memory then)
+cudaError_t decode_load(int precision);
 template <typename T>
 cudaError_t launch_decode(const DecodeArgs<T>& a, int grid, cudaStream_t stream);
 

@@ -18,3 +18,35 @@ def test_lone_frames_equal_the_full_device(cb, bg, z, n, rule, alpha):
         full = g.run_frames(3, "lone", 0, 0, n, 1.2, 4)
         assert np.array_equal(g.run_frames(3, "lone", 0, 0, 40, 1.2, 4), full[:40])
         assert np.array_equal(g.run_frames(3, "lone", 0, 50, 1, 1.2, 4), full[50:51])
+
+
+def test_no_alloc_calls_after_the_first_map_no_kernel(cb):
+    # One call on a small code loads all of the f64 decoder's builds: calls on the other base
+    # graph, with few and with many codewords, leave the free device memory as it was, and
+    # decide as the allocating decoder.
+    import ctypes as C
+
+    import torch
+
+    def setup(bg, z, n):
+        k, e = (22 if bg == 1 else 10) * z, (44 if bg == 1 else 20) * z
+        code = cb.NrLdpc(k, e, base_graph=bg, lifting_size=z, precision="f64")
+        gen = cb.NrLdpc(k, e, base_graph=bg, lifting_size=z, precision="f64")
+        llr = torch.from_numpy(gen.generate_frames(7, "no_alloc_f64", 0, 0, n, 1.0, 4)[0]).cuda()
+        out = [torch.full((n, (k + 31) // 32), -1, dtype=torch.int32, device="cuda") for _ in range(2)]
+        its = [torch.full((n,), -1, dtype=torch.int32, device="cuda") for _ in range(2)]
+        return code, gen, llr, out, its
+
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    L, ptr = cb.lib(), (lambda t: C.c_void_p(t.data_ptr()))
+    cases = [setup(2, 52, 4), setup(1, 36, 4), setup(1, 36, 2500), setup(2, 52, 2500)]
+    torch.cuda.synchronize()
+    for i, (code, _, llr, out, its) in enumerate(cases):
+        free = torch.cuda.mem_get_info()[0]
+        assert L.cb_decode_device_noalloc(code._h, ptr(llr), len(llr), ptr(out[0]), ptr(its[0]), stream) == 0
+        torch.cuda.synchronize()
+        assert i == 0 or torch.cuda.mem_get_info()[0] == free, i
+    for code, gen, llr, out, its in cases:
+        assert L.cb_decode_device(gen._h, ptr(llr), len(llr), ptr(out[1]), None, ptr(its[1]), stream) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(out[0], out[1]) and torch.equal(its[0], its[1])
