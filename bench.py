@@ -420,8 +420,8 @@ SPEC_WORKLOAD = ("specs/bicm_ldpc.yaml link: PEG(1024, 512) var degree 3 seed 1,
 # n f64 posteriors out, a 4-byte iteration count
 SPEC_ALGO_BYTES = SPEC_N * 8 * 2 + 4
 # dram__bytes_read.sum + dram__bytes_write.sum of one f64 decode of 2048 trials at 2.5 dB
-# (profiles/spec_link_sparse.md: 141,528,576 + 90,683,392 B)
-SPEC_TRAFFIC = 141_528_576 + 90_683_392
+# (profiles/spec_link_sparse.md: 141,240,832 + 88,792,064 B)
+SPEC_TRAFFIC = 141_240_832 + 88_792_064
 
 
 def spec_cpu_sample(steps, warmup, threads=0, budget_s=2.0):
@@ -556,8 +556,7 @@ def run_spec_ours(args, rank, world, local_rank):
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": SPEC_TRAFFIC, "traffic_source": "ncu capture of one f64 decode of 2048 trials at 2.5 dB "
                                                           "(bench.py --workload spec --profile-case --trials 2048)",
-                "kernel": "sparse_group_kernel<double, sum-product, register rows> (generic decoder, several codewords "
-                          "per CTA)",
+                "kernel": "sparse_edges_kernel<double> (generic decoder, an edge per thread, several codewords per CTA)",
                 "algorithmic_bytes_per_launch": T * SPEC_BLOCKS * SPEC_ALGO_BYTES, "launch_ms": dec,
                 "mean_iterations": float(iters.float().mean()),
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6.8 TB/s",
@@ -604,8 +603,8 @@ def run_spec_ours(args, rank, world, local_rank):
 
 MIX_N, MIX_ITEMS_SEED, MIX_SEED, MIX_NAME = 16384, 2024, 7, "bicm_ldpc_mix"
 # dram__bytes_read.sum + dram__bytes_write.sum of the decode phase of one replay
-# (profiles/mix_decode.md: 289,709,056 + 17,732,096 B)
-MIX_TRAFFIC = 289_709_056 + 17_732_096
+# (profiles/mix_decode.md: 290,579,456 + 19,790,592 B)
+MIX_TRAFFIC = 290_579_456 + 19_790_592
 MIX_METRIC = "decoded info Gbit/s of the uneven mixed batch (one graph replay per step); vs CPU Runner"
 MIX_WORKLOAD = ("16,384 codewords per replay, each: BG {1,2}, Z {16,32,64,128,208,384}, R {1/3,1/2,2/3,5/6}, "
                 "Gray QPSK..256-QAM, Eb/N0 U[0,6] dB (item seed 2024); f32, layered NMS alpha=0.75, <=25 "
@@ -766,9 +765,9 @@ LEARNED_POINTS = {"c5": {"learned": 6.97, "plain_20": 6.51, "plain_T": 7.33},
                   "c4": {"learned": 2.17, "plain_20": 2.09, "plain_T": 2.35}}
 LEARNED_FRAMES = {"c5": 8192, "c4": 65536}
 # dram__bytes_read.sum + dram__bytes_write.sum of one decode of a step's frames
-# (profiles/learned_decode_c5.md: 554,217,728 + 61,175,808 B; C4, the table-driven kernel: 272,915,712 +
-# 2,977,024 B)
-LEARNED_TRAFFIC = {"c5": 554_217_728 + 61_175_808, "c4": 272_915_712 + 2_977_024}
+# (profiles/learned_decode_c5.md: 556,848,128 + 3,322,368 B; C4, the table-driven kernel: 273,169,408 +
+# 3,445,504 B)
+LEARNED_TRAFFIC = {"c5": 556_848_128 + 3_322_368, "c4": 273_169_408 + 3_445_504}
 LEARNED_METRIC = "decoded info Gbit/s at equal FER (1e-3), neural vs plain min-sum; vs CPU Runner"
 
 
