@@ -61,7 +61,8 @@ bool build_nr_code(const CodeSpec& spec, NrCode& out, std::string& err);
 // their own column's posteriors from the others' when a syndrome test needs them.  At rate
 // 1/2 that leaves 24 of base graph 1's 46 rows (210 of 316 entries) and 12 of base graph 2's
 // 42 (77 of 197); the uneven mix of rates 1/3 to 5/6 decodes 16384 codewords in 9.0 instead of
-// 17.4 ms (8.0 with mix.cu's compile-time rows), 4096 f64 frames of BG2 Z = 52 at rate 1/2 in 1.3 instead of 2.8 ms.
+// 17.4 ms (8.0 with mix.cu's compile-time rows), 4096 f64 frames of BG2 Z = 52 at rate 1/2
+// in 1.3 instead of 2.8 ms.
 int live_rows(const NrCode& h);
 
 // xoshiro256** jump-ahead: the polynomial x^n mod P(x), P the characteristic
