@@ -587,14 +587,21 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
     }
     __syncthreads();
     const Tape cur(a.tape + (size_t)f * a.tape_frame + (size_t)t * a.tape_iter, lifted);
-    // the next row's record is loaded a row ahead
-    float2 n = make_float2(0.f, 0.f);
-    uint32_t nm = 0;
-    if (active) {
-      const int i = c.layer_order[run - 1] * z + tid;
-      n = cur.mag[i];
-      nm = cur.meta[i];
-    }
+    // the next row's record is loaded a row ahead: zeros for a skipped row that shares the last
+    // live level, whose record the forward pass does not write in every iteration (the
+    // level's sums form 0 times the record's magnitudes, NaN if they were infinite)
+    float2 n;
+    uint32_t nm;
+    auto record = [&](int q, float2& mag, uint32_t& meta) {
+      mag = make_float2(0.f, 0.f);
+      meta = 0;
+      const int L = c.layer_order[q];
+      if (active && L < live) {
+        mag = cur.mag[L * z + tid];
+        meta = cur.meta[L * z + tid];
+      }
+    };
+    record(run - 1, n, nm);
     // the skipped rows, the last of the forward pass
     if constexpr (SHARED) {
       if (own_loss && (multi || t == a.T - 1)) buf = own_columns_bwd(a, gp, cur, live, t, wbuf, red, buf);
@@ -607,11 +614,7 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
         const int s0 = c.layer_start[L], d = c.layer_start[L + 1] - s0;
         float2 nn = n;
         uint32_t nmn = nm;
-        if (active && qe > 0) {
-          const int i = c.layer_order[qe - 1] * z + tid;
-          nn = cur.mag[i];
-          nmn = cur.meta[i];
-        }
+        if (qe > 0) record(qe - 1, nn, nmn);
         float* rd = red + ((size_t)buf * nw + warp) * RW + 2 * at;
 #define CB_ROW(DD)                                                                                                 \
   learned_row_bwd<DD, SHARED, S>(a, gp, gc + (size_t)s0 * S, n, nm, t, s0, tid, z, active && L < live, t == a.T - 1, w, rd, lane);
