@@ -582,7 +582,7 @@ cb_status cb_code_create(const cb_code_desc* d, cb_code** out) {
   c->cfg.layered = d->layered;
   c->cfg.max_iterations = d->max_iterations;
   cbk::fill_dev_code(c->host, c->dev);
-  cbk::set_live_rows(c->dev, cbk::decoder_rows(c->host, d->alpha));
+  cbk::set_live_rows(c->dev, cbk::decoder_rows(c->host, d->rule, d->alpha));
   if (d->rule == CB_RULE_SUM_PRODUCT || !d->layered) {
     // lifted row (L, r) holds, for the entries (j, s) of base row L in table order, the
     // variable j Z + (r + s) mod Z (nr/ldpc.rs:124-134)
@@ -845,6 +845,8 @@ struct cb_nms {
   float* d_v = nullptr;
   unsigned char* d_tape = nullptr;
   size_t tape_cap = 0;
+  int32_t* d_live = nullptr;
+  size_t live_cap = 0;
   float* d_P = nullptr;
   size_t P_cap = 0;
   float* d_c2v = nullptr;
@@ -877,8 +879,10 @@ cb_status nms_buffers(cb_nms* h, int64_t n, NmsUse use) {
   CB_CUDA(c, grow(h->d_post, h->post_cap, (size_t)n * c->host.n_full * 4));
   CB_CUDA(c, grow(h->d_info, h->info_cap, (size_t)n * ((c->host.k_info + 31) / 32) * 4));
   CB_CUDA(c, grow(h->d_res, h->res_cap, (size_t)n * sizeof(cbd::FrameResult)));
-  if (use != kNmsEvaluate)
+  if (use != kNmsEvaluate) {
+    CB_CUDA(c, grow(h->d_live, h->live_cap, (size_t)n * 4));
     CB_CUDA(c, grow(h->d_tape, h->tape_cap, (size_t)n * (use == kNmsTrain ? h->T : 1) * cbk::learned_tape_bytes(c->dev)));
+  }
   if (use == kNmsTrain) {
     CB_CUDA(c, grow(h->d_c2v, h->c2v_cap, (size_t)n * c->dev.n_entries * cbk::learned_stride(c->dev) * 4));
     CB_CUDA(c, grow(h->d_P, h->P_cap, (size_t)n * h->T * c->host.n_full * 4));
@@ -923,15 +927,19 @@ int nms_nr_grid(cb_nms* h) {
 
 // The base rows that evaluation runs: as the plain decoder (cbh::live_rows) when the skipped
 // rows' messages are zero, max(alpha 0 - beta, 0), so no offset of theirs but the own
-// column's is negative.  Needs the host copy of the weights.
+// column's is negative, and the own column's weights keep its messages finite.  Needs the
+// host copy of the weights (learned_live_kernel tests the same on the device).
 int nms_live_rows(const cb_nms* h) {
   const cbh::NrCode& c = h->code->host;
   const int live = cbh::live_rows(c), ne = (int)c.entry_col.size();
-  const float* beta = h->h_w.data() + h->nw;
+  const float *alpha = h->h_w.data(), *beta = alpha + h->nw;
   for (int t = 0; t < h->T; t++)
-    for (int L = live; L < c.rows_n; L++)
+    for (int L = live; L < c.rows_n; L++) {
+      const size_t w = (size_t)t * ne, own = w + c.layer_start[L + 1] - 1;
       for (int e = c.layer_start[L]; e + 1 < c.layer_start[L + 1]; e++)
-        if (beta[(size_t)t * ne + e] < 0.f) return c.rows_n;
+        if (beta[w + e] < 0.f) return c.rows_n;
+      if (!cbd::skippable_own_weights(alpha[own], beta[own])) return c.rows_n;
+    }
   return live;
 }
 
@@ -1027,6 +1035,7 @@ cbk::LearnedArgs nms_args(cb_nms* h, int64_t n) {
   a.code = h->code->dev;
   cbk::set_live_rows(a.code, cbh::live_rows(h->code->host));
   a.live = reinterpret_cast<int32_t*>(h->d_loss) + 1;
+  a.frame_live = h->d_live;
   a.T = h->T;
   a.shared = h->shared;
   a.alpha = h->d_w;
@@ -1101,7 +1110,7 @@ void cb_nms_destroy(cb_nms* h) {
   if (!h) return;
   cudaSetDevice(h->code->device);
   void* bufs[] = {h->d_w, h->d_g, h->d_m, h->d_v, h->d_tape, h->d_P, h->d_c2v, h->d_post, h->d_llr, h->d_cw, h->d_info,
-                  h->d_ebn0, h->d_loss, h->d_res, h->d_bytes};
+                  h->d_ebn0, h->d_loss, h->d_res, h->d_bytes, h->d_live};
   for (void* p : bufs)
     if (p) cudaFree(p);
   delete h;

@@ -259,7 +259,7 @@ cb_status cb_mix_create(const cb_mix_item* items, int64_t n, uint64_t seed, uint
   // update first, so that the last ones to be taken are short
   std::vector<int> work(m->codes.size());
   for (size_t i = 0; i < work.size(); i++)
-    work[i] = m->codes[i].layer_start[cbk::decoder_rows(m->codes[i], (double)m->alpha)];
+    work[i] = m->codes[i].layer_start[cbk::decoder_rows(m->codes[i], cbd::RULE_NMS, (double)m->alpha)];
   std::stable_sort(its.begin(), its.end(), [&](const cbk::MixItem& a, const cbk::MixItem& b) {
     const int za = m->codes[a.code].z, zb = m->codes[b.code].z;
     return za != zb ? za > zb : work[a.code] > work[b.code];
@@ -290,7 +290,7 @@ cb_status cb_mix_create(const cb_mix_item* items, int64_t n, uint64_t seed, uint
   m->dev_codes.resize(m->codes.size());
   for (size_t i = 0; i < m->codes.size(); i++) {
     cbk::fill_dev_code(m->codes[i], m->dev_codes[i]);
-    cbk::set_live_rows(m->dev_codes[i], cbk::decoder_rows(m->codes[i], (double)m->alpha));
+    cbk::set_live_rows(m->dev_codes[i], cbk::decoder_rows(m->codes[i], cbd::RULE_NMS, (double)m->alpha));
   }
   m->gen_smem = 0;
   for (auto& kv : config_id) {

@@ -315,6 +315,13 @@ int live_rows(const NrCode& h) {
     // (the own column is the row's last entry, as the tables list them)
     if (h.entry_col[h.layer_start[live] - 1] != col || degree[col] != 1) break;
     if (h.inv_start[(size_t)(col + 1) * h.z] != h.inv_start[(size_t)col * h.z]) break;  // some bit is sent
+    // (the columns whose magnitudes the decoders watch, beyond_skipping in dev_math.cuh)
+    bool watched = false;
+    for (int t = h.layer_start[live - 1]; t < h.layer_start[live]; t++) {
+      const int j = h.entry_col[t];
+      watched = watched || j < 2 || (h.bg == 2 && (j == 2 || j == 10));
+    }
+    if (!watched) break;
   }
   return live;
 }

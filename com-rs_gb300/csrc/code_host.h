@@ -58,7 +58,9 @@ bool build_nr_code(const CodeSpec& spec, NrCode& out, std::string& err);
 // iteration its row sends them zero and, its smallest incoming magnitude being theirs, every
 // other variable a message of magnitude alpha 0 (or max(0 - offset, 0)) = 0: the row changes
 // nothing but its own column.  No later row is live, so the decoders skip these rows, and form
-// their own column's posteriors from the others' when a syndrome test needs them.  At rate
+// their own column's posteriors from the others' when a syndrome test needs them.  A codeword
+// whose magnitudes approach infinity, where this no longer holds, is decoded again with every
+// row (beyond_skipping in dev_math.cuh).  At rate
 // 1/2 that leaves 24 of base graph 1's 46 rows (210 of 316 entries) and 12 of base graph 2's
 // 42 (77 of 197); the uneven mix of rates 1/3 to 5/6 decodes 16384 codewords in 9.0 instead of
 // 17.4 ms (8.0 with mix.cu's compile-time rows), 4096 f64 frames of BG2 Z = 52 at rate 1/2

@@ -61,17 +61,17 @@ enum LearnedWeights { kPlain = 0, kWeightsGlobal = 1, kWeightsParam = 2, kWeight
 template <typename T, int LW, int RULE, int MAXD, bool FULL>
 __device__ __forceinline__ void decode_layers(const cbd::DevCode& c, T* post, const StateSlot<T>& st,
                                               const LearnedRowW& lw, int iter, int tid, int z, bool active,
-                                              T alpha, const ScaleF64& scale) {
+                                              T alpha, const ScaleF64& scale, int run) {
   constexpr bool AHEAD = sizeof(T) == 8 && FULL;
   T b1 = (T)0, b2 = (T)0;
   uint32_t bt = 0;
   if (AHEAD && iter > 1 && active) st.load(c.layer_order[0] * z + tid, b1, b2, bt);
-  for (int q = 0; q < c.rows_run; q++) {
+  for (int q = 0; q < run; q++) {
     const int L = c.layer_order[q];
     T a1 = b1, a2 = b2;
     uint32_t mt = bt;
     if (AHEAD) {
-      if (iter > 1 && active && q + 1 < c.rows_run) st.load(c.layer_order[q + 1] * z + tid, b1, b2, bt);
+      if (iter > 1 && active && q + 1 < run) st.load(c.layer_order[q + 1] * z + tid, b1, b2, bt);
     } else if (iter > 1 && active) {
       st.load(L * z + tid, a1, a2, mt);
     }
@@ -121,13 +121,13 @@ __device__ __forceinline__ void row_positions(int (&off)[D], const cbd::DevCode&
 // 4.18 ms), so it keeps decode_layers.
 template <int BG, int RULE, int Q>
 __device__ __forceinline__ void decode_rows(const cbd::DevCode& c, double* post, const StateSlot<double>& st,
-                                            bool first, int r, int z, bool active, const ScaleF64& scale, double a1,
-                                            double a2, uint32_t mt) {
+                                            bool first, int r, int z, bool active, const ScaleF64& scale, int live,
+                                            double a1, double a2, uint32_t mt) {
   using G = cbn::Graph<BG>;
   if constexpr (Q < G::rows) {
     if constexpr (Q >= 4) {
       if constexpr (G::level_end[Q - 1] != 0) {
-        if (c.rows_live <= cbn::rest_min<BG>(Q)) return;
+        if (live <= cbn::rest_min<BG>(Q)) return;
       }
     }
     constexpr int L = G::order[Q], S0 = G::start[L], D = G::start[L + 1] - S0;
@@ -149,16 +149,16 @@ __device__ __forceinline__ void decode_rows(const cbd::DevCode& c, double* post,
       st.store(L * zz + rr, n1, n2, nm);
     }
     if constexpr (G::level_end[Q] != 0) __syncthreads();
-    decode_rows<BG, RULE, Q + 1>(c, post, st, first, r, z, active, scale, b1, b2, bt);
+    decode_rows<BG, RULE, Q + 1>(c, post, st, first, r, z, active, scale, live, b1, b2, bt);
   }
 }
 template <int BG, int RULE>
 __device__ __forceinline__ void decode_rows(const cbd::DevCode& c, double* post, const StateSlot<double>& st,
-                                            bool first, int r, int z, bool active, const ScaleF64& scale) {
+                                            bool first, int r, int z, bool active, const ScaleF64& scale, int live) {
   double a1 = 0.0, a2 = 0.0;
   uint32_t mt = 0u;
   if (active && !first) st.load(cbn::Graph<BG>::order[0] * z + r, a1, a2, mt);
-  decode_rows<BG, RULE, 0>(c, post, st, first, r, z, active, scale, a1, a2, mt);
+  decode_rows<BG, RULE, 0>(c, post, st, first, r, z, active, scale, live, a1, a2, mt);
 }
 
 template <typename T, int LW, int MAXD, bool FULL>
@@ -175,6 +175,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float*
   uint16_t* s_lstart = reinterpret_cast<uint16_t*>(s_ent + c.n_entries);
   __shared__ long long s_cw;
   __shared__ unsigned int s_err;
+  __shared__ int s_mode, s_beyond;  // as in layered_nr.cuh
   const int rows = c.rows_n * z;
   const StateSlot<T> st(reinterpret_cast<unsigned char*>(a.state) + (size_t)blockIdx.x * slot_bytes<T>(rows), rows);
   const T alpha = (T)a.cfg.alpha;
@@ -186,9 +187,16 @@ __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float*
   for (int i = tid; i < c.n_entries; i += nt) s_ent[i] = c.entry[i];
   for (int i = tid; i <= c.rows_n; i += nt) s_lstart[i] = c.layer_start[i];
 
+  if (tid == 0) s_mode = 0;
   for (;;) {
     if (tid == 0) {
-      s_cw = (long long)atomicAdd(reinterpret_cast<unsigned long long*>(a.work_counter), 1ull);
+      if (s_mode == cbn::kAgain) {
+        s_mode = cbn::kEveryRow;
+      } else {
+        s_mode = 0;
+        s_cw = (long long)atomicAdd(reinterpret_cast<unsigned long long*>(a.work_counter), 1ull);
+      }
+      s_beyond = 0;
       s_err = 0;
     }
     __syncthreads();
@@ -199,6 +207,12 @@ __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float*
     const T* llr = a.llr + (size_t)cw * c.e;
     for (int v = tid; v < c.n_full; v += nt) post[v] = (T)0;
     __syncthreads();
+    Widest<T> widest;
+    auto put = [&](T* d, T l) {
+      const T v = add_rn((T)0, l);
+      widest.add(v);
+      *d = v;
+    };
     if (c.map_is_offset) {
       if (sizeof(T) == 4 && (c.e & 3) == 0 && (reinterpret_cast<uintptr_t>(a.llr) & 15) == 0) {
         // 128-bit streaming loads: a 16-byte aligned buffer with E % 4 == 0 keeps every
@@ -207,26 +221,29 @@ __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float*
         for (int q = tid; q < (c.e >> 2); q += nt) {
           const float4 v = __ldcs(l4 + q);
           T* d = post + 2 * z + 4 * q;
-          d[0] = add_rn((T)0, (T)v.x);
-          d[1] = add_rn((T)0, (T)v.y);
-          d[2] = add_rn((T)0, (T)v.z);
-          d[3] = add_rn((T)0, (T)v.w);
+          put(d, (T)v.x);
+          put(d + 1, (T)v.y);
+          put(d + 2, (T)v.z);
+          put(d + 3, (T)v.w);
         }
       } else {
-        for (int t = tid; t < c.e; t += nt) post[2 * z + t] = add_rn((T)0, __ldcs(llr + t));
+        for (int t = tid; t < c.e; t += nt) put(post + 2 * z + t, __ldcs(llr + t));
       }
     } else if (!c.has_repeats) {
-      for (int t = tid; t < c.e; t += nt) post[c.map[t]] = add_rn((T)0, __ldcs(llr + t));
+      for (int t = tid; t < c.e; t += nt) put(post + c.map[t], __ldcs(llr + t));
     } else {
       for (int v = tid; v < c.n_full; v += nt) {
         int b0 = c.inv_start[v], b1 = c.inv_start[v + 1];
         if (b0 == b1) continue;
         T s = (T)0;
         for (int i = b0; i < b1; i++) s = add_rn(s, llr[c.inv_t[i]]);
-        post[v] = s;
+        put(post + v, s);
       }
     }
+    if (widest.beyond()) s_mode = cbn::kEveryRow;
     __syncthreads();
+    const bool every = s_mode == cbn::kEveryRow;
+    const int live = every ? c.rows_n : c.rows_live;
     for (int v = c.k_info + tid; v < c.k; v += nt) post[v] = (T)cbd::kKnownBitLlr;
     __syncthreads();
 
@@ -270,28 +287,40 @@ __device__ __forceinline__ void decode_body(const DecodeArgs<T>& a, const float*
         if constexpr (sizeof(T) == 8 && !FULL) {
           constexpr int BG = MAXD == 19 ? 1 : 2;
           if (rule == cbd::RULE_NMS)
-            decode_rows<BG, cbd::RULE_NMS>(c, post, st, iter == 1, tid, z, active, scale);
+            decode_rows<BG, cbd::RULE_NMS>(c, post, st, iter == 1, tid, z, active, scale, live);
           else
-            decode_rows<BG, cbd::RULE_OMS>(c, post, st, iter == 1, tid, z, active, scale);
+            decode_rows<BG, cbd::RULE_OMS>(c, post, st, iter == 1, tid, z, active, scale, live);
         } else if (LEARNED || rule == cbd::RULE_NMS)
-          decode_layers<T, LW, cbd::RULE_NMS, MAXD, FULL>(c, post, st, lw, iter, tid, z, active, alpha, scale);
+          decode_layers<T, LW, cbd::RULE_NMS, MAXD, FULL>(c, post, st, lw, iter, tid, z, active, alpha, scale,
+                                                          every ? c.rows_n : c.rows_run);
         else
-          decode_layers<T, LW, cbd::RULE_OMS, MAXD, FULL>(c, post, st, lw, iter, tid, z, active, alpha, scale);
+          decode_layers<T, LW, cbd::RULE_OMS, MAXD, FULL>(c, post, st, lw, iter, tid, z, active, alpha, scale,
+                                                          every ? c.rows_n : c.rows_run);
         // the skipped rows' own columns (formed for the full syndrome test only)
         auto own = [&]() {
-          if (c.rows_live == c.rows_n) return;
-          unsent_rows(post, s_ent, s_lstart, c.rows_live, c.rows_n, z, tid, nt,
+          if (live == c.rows_n) return;
+          unsent_rows(post, s_ent, s_lstart, live, c.rows_n, z, tid, nt,
                       [w_ac, w_bc, w_stride, z, rule, alpha](int e, int r, T m) -> T {
             if constexpr (LEARNED) return LearnedRowW::mag_at(w_ac, w_bc, w_stride == 1 ? e : e * z + r, m);
             else return rule == cbd::RULE_NMS ? mul_rn(alpha, m) : (T)fmax(sub_rn(m, alpha), (T)0);
           });
           __syncthreads();
         };
+        if (LEARNED && live < c.rows_n && active && beyond_skipping(post, tid, z, c.bg)) s_beyond = 1;
         if (!some_check_fails_after(post, hd, s_ent, s_lstart, c.rows_n, ncol, z, tid, nt, own)) {
           it = iter;
           break;
         }
         if (LEARNED && iter == max_it && a.post_out) own();  // (the whole word's posteriors go out)
+      }
+      if (live < c.rows_n) {
+        if (active && beyond_skipping(post, tid, z, c.bg)) s_beyond = 1;
+        __syncthreads();
+        if (s_beyond) {
+          __syncthreads();
+          if (tid == 0) s_mode = cbn::kAgain;
+          continue;
+        }
       }
     }
 

@@ -59,10 +59,10 @@ inline void fill_dev_code(const cbh::NrCode& h, cbd::DevCode& v) {
   v.rows_live = v.rows_run = h.rows_n;
 }
 
-// the base rows that a min-sum decoder runs: with a scale or offset that is negative or not
-// finite none is skipped
-inline int decoder_rows(const cbh::NrCode& h, double alpha) {
-  return alpha >= 0 && std::isfinite(alpha) ? cbh::live_rows(h) : h.rows_n;
+// the base rows that a min-sum decoder runs: none is skipped with a scale or offset that is
+// negative or not finite, or a scale above 1 (beyond_skipping)
+inline int decoder_rows(const cbh::NrCode& h, int rule, double alpha) {
+  return alpha >= 0 && std::isfinite(alpha) && (rule == cbd::RULE_OMS || alpha <= 1) ? cbh::live_rows(h) : h.rows_n;
 }
 
 // the schedule of the rows before `live`: whole levels

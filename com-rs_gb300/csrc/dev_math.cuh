@@ -157,6 +157,46 @@ __device__ __forceinline__ bool some_check_fails_after(const T* post, uint32_t* 
   return some_packed_check_fails(post, hd, ent, lstart, rows_n, ncol, z, tid, nt);
 }
 
+// Magnitudes beyond which a codeword runs every row: those in which a skipped row may change
+// more than its own column.  Such a row sends zero because its own variable comes in with
+// magnitude zero, what the row made of it less its old message, while that is finite: from
+// an infinite one inf - inf is NaN, which the minimum passes over, and the row's other
+// variables get messages.  Every skipped row has an edge in one of the watched base columns
+// (0 and 1, in base graph 2 also 2 and 10; cbh::live_rows asks for it), so its smallest magnitude
+// is finite while those columns are.  A posterior that is not finite never is again, so the plain
+// rules, which make no magnitude larger (cbk::decoder_rows), are tested at a codeword's end; a
+// learned scale may (up to cbd::kSkipMaxScale), so there the test follows every iteration.
+// A codeword that fails it is decoded again.  The channel LLRs are tested where they are
+// loaded: infinite ones end in the watched columns anyway, and beside a NaN the pairwise
+// minimum search finds another second minimum.  (Tested after every iteration the plain
+// decoders took 1-2 % longer.)
+__device__ __forceinline__ bool beyond_skipping(float v) { return (__float_as_uint(v) & 0x7fffffffu) >= (127u + 100u) << 23; }
+__device__ __forceinline__ bool beyond_skipping(double v) {
+  return ((uint32_t)__double2hiint(v) & 0x7fffffffu) >= (1023u + 1000u) << 20;
+}
+// the watched variables of lifted row r
+template <typename T>
+__device__ __forceinline__ bool beyond_skipping(const T* post, int r, int z, int bg) {
+  return beyond_skipping(post[r]) || beyond_skipping(post[z + r]) ||
+         (bg == 2 && (beyond_skipping(post[2 * z + r]) || beyond_skipping(post[10 * z + r])));
+}
+// whether some of a thread's values is beyond the bound, an instruction a value in f32
+// (tested one by one the loads of a rate 1/2 codeword took 1 % of its decoding)
+template <typename T>
+struct Widest;
+template <>
+struct Widest<float> {
+  float most = 0.0f;
+  __device__ __forceinline__ void add(float v) { asm("max.NaN.f32 %0, %0, %1;" : "+f"(most) : "f"(fabsf(v))); }
+  __device__ __forceinline__ bool beyond() const { return beyond_skipping(most); }
+};
+template <>
+struct Widest<double> {
+  bool some = false;
+  __device__ __forceinline__ void add(double v) { some = some || beyond_skipping(v); }
+  __device__ __forceinline__ bool beyond() const { return some; }
+};
+
 // The own parity columns of the base rows [live, rows): columns that are not sent and in no
 // other row (cbh::live_rows).  What such a row makes of its variable is 0 + the message
 // from the row's other variables, whose messages from the row are zero: their smallest
@@ -174,7 +214,7 @@ __device__ __forceinline__ void unsent_rows(T* post, const uint32_t* ent, const 
       int cc = r + (int)(en & 0xffffu);
       cc -= (cc >= z) ? z : 0;
       const T v = post[(int)(en >> 16) * z + cc];
-      neg ^= (uint32_t)(v < (T)0);
+      neg ^= is_negative(v);
       m = fmin(m, fabs(v));
     }
     const uint32_t en = ent[own];

@@ -75,6 +75,15 @@ struct FrameResult {
   uint16_t reserved;
 };
 
+// The learned scale up to which the magnitudes of skipped rows (cbh::live_rows) stay finite
+// below the bound of beyond_skipping (dev_math.cuh).
+constexpr float kSkipMaxScale = 1048576.0f;
+
+// whether a skipped row's own column may have these learned weights: scale m - offset stays finite
+__host__ __device__ inline bool skippable_own_weights(float scale, float offset) {
+  return scale <= kSkipMaxScale && scale >= -kSkipMaxScale && offset >= -kSkipMaxScale;
+}
+
 constexpr float kKnownBitLlr = 30.0f;  // KNOWN_BIT_LLR, crates/com-core/src/signal.rs:37
 
 }  // namespace cbd

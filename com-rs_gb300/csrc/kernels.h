@@ -187,7 +187,10 @@ struct LearnedArgs {
   int32_t loss_bits;        // the loss covers codeword bits [0, loss_bits): n_full, or K' (the information bits)
   float* g_alpha;           // gradients of the mean loss (backward)
   float* g_beta;
-  int32_t* live;            // shared weights: the rows that the passes run, set by the forward launch
+  // shared weights, set by the forward launch: the rows that the weights allow the passes to
+  // run, and [n_frames] those that each frame ran
+  int32_t* live;
+  int32_t* frame_live;
 };
 // from one base-graph entry's message gradients to the next's: a compile-time constant of
 // the backward kernels

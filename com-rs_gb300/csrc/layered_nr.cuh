@@ -350,6 +350,10 @@ __host__ __device__ constexpr int rest_min(int q) {
   return m;
 }
 
+// the marks of a codeword that runs every row, and of one that has to be decoded again so
+// (beyond_skipping)
+constexpr int kEveryRow = 2, kAgain = 1;
+
 struct NrState {
   unsigned char* mag;
   unsigned char* meta;
@@ -407,13 +411,14 @@ __device__ __forceinline__ void nr_dense_rows_bg1(unsigned char* post, const NrA
 template <int BG, class K, int Q, int RULE, class W>
 __device__ __forceinline__ void nr_iteration(unsigned char* post, const NrArgs& a, const NrState& st, int r, int r4,
                                              int z4, int z, bool active, bool first, float alpha, const W& w,
-                                             float a1, float a2, uint32_t mt, float b1, float b2, uint32_t bt) {
+                                             float a1, float a2, uint32_t mt, float b1, float b2, uint32_t bt,
+                                             const int& mode) {
   if constexpr (Q < Graph<BG>::rows) {
     // at a level's start: every row from here on changes only its own column, which is not
-    // sent (the syndrome test forms it)
+    // sent (the syndrome test forms it), unless the codeword runs every row
     if constexpr (K::prune && Q >= 4) {
       if constexpr (Graph<BG>::level_end[Q - 1] != 0) {
-        if (a.live <= rest_min<BG>(Q)) return;
+        if (a.live <= rest_min<BG>(Q) && mode != kEveryRow) return;
       }
     }
     constexpr int L = Graph<BG>::order[Q];
@@ -444,7 +449,7 @@ __device__ __forceinline__ void nr_iteration(unsigned char* post, const NrArgs& 
       st.store(L * zz + rr, n1, n2, nm);
     }
     if constexpr (Graph<BG>::level_end[Q] != 0) __syncthreads();
-    nr_iteration<BG, K, Q + 1, RULE>(post, a, st, r, r4, z4, z, active, first, alpha, w, b1, b2, bt, c1, c2, ct);
+    nr_iteration<BG, K, Q + 1, RULE>(post, a, st, r, r4, z4, z, active, first, alpha, w, b1, b2, bt, c1, c2, ct, mode);
   }
 }
 
@@ -515,6 +520,8 @@ __global__ void __launch_bounds__(384, 2) layered_nr_kernel(const __grid_constan
   uint16_t* s_lstart = reinterpret_cast<uint16_t*>(s_ent + a.n_entries);
   __shared__ long long s_cw;
   __shared__ unsigned int s_err;
+  __shared__ int s_mode;    // kEveryRow: the codeword runs every row; kAgain: it has to be decoded again so
+  __shared__ int s_beyond;  // some magnitude was beyond_skipping
   const int lifted = a.rows * z;
   unsigned char* slot = a.state + (size_t)blockIdx.x * nr_state_bytes(lifted);
   const NrState st{slot, slot + (size_t)lifted * 8, l2_evict_last_policy()};
@@ -529,7 +536,7 @@ __global__ void __launch_bounds__(384, 2) layered_nr_kernel(const __grid_constan
 
   // the posteriors of the skipped rows' own columns after iteration `iter`
   auto own_columns = [&](int iter) {
-    if (a.live == a.rows) return;
+    if (a.live == a.rows || s_mode == kEveryRow) return;
     const auto w = wset.staged(iter - 1);
     unsent_rows_call(post, s_ent, s_lstart, a.live, a.rows, z, tid, nt, [w, nms, alpha](int e, int, float m) {
       if constexpr (decltype(w)::learned) return learned_mag(w.ac(e), w.bc(e), m);
@@ -538,9 +545,16 @@ __global__ void __launch_bounds__(384, 2) layered_nr_kernel(const __grid_constan
     __syncthreads();
   };
 
+  if (tid == 0) s_mode = 0;
   for (;;) {
     if (tid == 0) {
-      s_cw = (long long)atomicAdd(a.work_counter, 1ull);
+      if (K::prune && s_mode == kAgain) {
+        s_mode = kEveryRow;
+      } else {
+        s_mode = 0;
+        s_cw = (long long)atomicAdd(a.work_counter, 1ull);
+      }
+      s_beyond = 0;
       s_err = 0;
     }
     __syncthreads();
@@ -552,31 +566,38 @@ __global__ void __launch_bounds__(384, 2) layered_nr_kernel(const __grid_constan
     const float* llr = a.llr + (size_t)cw * a.e;
     for (int v = tid; v < n_full; v += nt) post[v] = 0.0f;
     __syncthreads();
+    Widest<float> widest;
+    auto put = [&](float* d, float l) {
+      const float v = __fadd_rn(0.0f, l);
+      if constexpr (K::prune) widest.add(v);
+      *d = v;
+    };
     if (a.map_kind == 0) {
       if ((a.e & 3) == 0 && (reinterpret_cast<uintptr_t>(a.llr) & 15) == 0) {
         const float4* l4 = reinterpret_cast<const float4*>(llr);
         for (int q = tid; q < (a.e >> 2); q += nt) {
           const float4 v = __ldcs(l4 + q);
           float* d = post + 2 * z + 4 * q;
-          d[0] = __fadd_rn(0.0f, v.x);
-          d[1] = __fadd_rn(0.0f, v.y);
-          d[2] = __fadd_rn(0.0f, v.z);
-          d[3] = __fadd_rn(0.0f, v.w);
+          put(d, v.x);
+          put(d + 1, v.y);
+          put(d + 2, v.z);
+          put(d + 3, v.w);
         }
       } else {
-        for (int t = tid; t < a.e; t += nt) post[2 * z + t] = __fadd_rn(0.0f, __ldcs(llr + t));
+        for (int t = tid; t < a.e; t += nt) put(post + 2 * z + t, __ldcs(llr + t));
       }
     } else if (a.map_kind == 1) {
-      for (int t = tid; t < a.e; t += nt) post[a.map[t]] = __fadd_rn(0.0f, __ldcs(llr + t));
+      for (int t = tid; t < a.e; t += nt) put(post + a.map[t], __ldcs(llr + t));
     } else {
       for (int v = tid; v < n_full; v += nt) {
         const int b0 = a.inv_start[v], b1 = a.inv_start[v + 1];
         if (b0 == b1) continue;
         float s = 0.0f;
         for (int i = b0; i < b1; i++) s = __fadd_rn(s, llr[a.inv_t[i]]);
-        post[v] = s;
+        put(post + v, s);
       }
     }
+    if (K::prune && widest.beyond()) s_mode = kEveryRow;
     __syncthreads();
     for (int v = a.k_info + tid; v < a.k; v += nt) post[v] = 30.0f;  // KNOWN_BIT_LLR, signal.rs:37
     __syncthreads();
@@ -605,7 +626,7 @@ __global__ void __launch_bounds__(384, 2) layered_nr_kernel(const __grid_constan
             st.load(Graph<BG>::order[5] * z + tid, b1, b2, bt);
           }
           nr_iteration<BG, K, 4, K::rule>(pb, a, st, tid, r4, z4, z, active, iter == 1, alpha, w, a1, a2, mt, b1, b2,
-                                          bt);
+                                          bt, s_mode);
         } else {
         if constexpr (NrTuning<K>::ahead == 2) {
           if (active && iter != 1) {
@@ -618,19 +639,33 @@ __global__ void __launch_bounds__(384, 2) layered_nr_kernel(const __grid_constan
         // both rules' magnitudes in every row: 14.7 against 14.2 ms per 8192 C2 codewords)
         if constexpr (K::rule != 0) {
           nr_iteration<BG, K, 0, K::rule>(pb, a, st, tid, r4, z4, z, active, iter == 1, alpha, wset.at(iter - 1), a1,
-                                          a2, mt, b1, b2, bt);
+                                          a2, mt, b1, b2, bt, s_mode);
         } else if (nms) {
           nr_iteration<BG, K, 0, 1>(pb, a, st, tid, r4, z4, z, active, iter == 1, alpha, wset.at(iter - 1), a1, a2, mt,
-                                    b1, b2, bt);
+                                    b1, b2, bt, s_mode);
         } else {
           nr_iteration<BG, K, 0, 2>(pb, a, st, tid, r4, z4, z, active, iter == 1, alpha, wset.at(iter - 1), a1, a2, mt,
-                                    b1, b2, bt);
+                                    b1, b2, bt, s_mode);
         }
+        }
+        if constexpr (K::prune && decltype(wset)::learned) {
+          if (active && beyond_skipping(post, tid, z, BG)) s_beyond = 1;
         }
         if (!some_nr_check_fails<BG, K>(post, hd, s_ent, s_lstart, a, ncol, z, tid, nt, r4, z4,
                                         [&] { own_columns(iter); })) {
           it = iter;
           break;
+        }
+      }
+      if constexpr (K::prune) {
+        if (a.live < a.rows) {
+          if (active && beyond_skipping(post, tid, z, BG)) s_beyond = 1;
+          __syncthreads();
+          if (s_beyond && s_mode != kEveryRow) {
+            __syncthreads();
+            if (tid == 0) s_mode = kAgain;
+            continue;
+          }
         }
       }
     }

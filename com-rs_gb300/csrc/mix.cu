@@ -114,8 +114,10 @@ __device__ __forceinline__ void mix_rows(unsigned char* post, const MixTable& ta
 }
 
 // Decode one codeword of the batch in a slot; RHO rows per thread (0: one, by mix_rows).
+// flag[0] is slot_any's; flag[1] is set when the codeword runs every row (beyond_skipping).
+// Returns whether the codeword has to be decoded again so.
 template <int RHO>
-__device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned char* sm, int ncol_max,
+__device__ bool decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned char* sm, int ncol_max,
                             const StateSlot<float>& st, int lt, int nt, int bar, int* flag, unsigned int* err) {
   const cbd::DevCode& c = a.codes[it.code];
   const int z = c.z;
@@ -139,17 +141,25 @@ __device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned 
     s_end[i] = c.level_end[i];
   }
   const float* llr = a.llr + it.llr_offset;
+  const int rule = a.rule;
+  const float alpha = a.alpha;
+  const int rows_n = c.rows_n;
+  volatile int* every = flag + 1;
   for (int v = lt; v < c.n_full; v += nt) post[v] = 0.f;
   slot_sync(bar, nt);
   // the batch's codes all use the plain rate matching 2Z + t
-  for (int t = lt; t < c.e; t += nt) post[2 * z + t] = __fadd_rn(0.f, __ldcs(llr + t));
+  Widest<float> widest;
+  for (int t = lt; t < c.e; t += nt) {
+    const float v = __fadd_rn(0.f, __ldcs(llr + t));
+    widest.add(v);
+    post[2 * z + t] = v;
+  }
+  if (widest.beyond()) *every = 1;
   slot_sync(bar, nt);
+  const int rows_run = *every ? rows_n : c.rows_run, rows_live = *every ? rows_n : c.rows_live;
   for (int v = c.k_info + lt; v < c.k; v += nt) post[v] = cbd::kKnownBitLlr;
   slot_sync(bar, nt);
   int iters = 0;
-  const int rule = a.rule;
-  const float alpha = a.alpha;
-  const int rows_n = c.rows_n, rows_run = c.rows_run, rows_live = c.rows_live;
   if (slot_check_fails(post, hd, s_ent, s_lstart, rows_n, ncol, z, lt, nt, bar, flag, [] {})) {
     iters = a.max_it;
     for (int iter = 1; iter <= a.max_it; iter++) {
@@ -193,6 +203,14 @@ __device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned 
         break;
       }
     }
+    if (rows_live < rows_n) {
+      int beyond = 0;
+      for (int r = lt; r < z; r += nt) beyond |= (int)beyond_skipping(post, r, z, c.bg);
+      if (slot_any(beyond, flag, bar, nt, lt)) {
+        if (lt == 0) *every = 1;
+        return true;
+      }
+    }
   }
   // counts against the sent info bits: the sent words, one per thread, loaded before the
   // ballots so that their latency overlaps them, against the decisions staged in hd (free
@@ -218,17 +236,19 @@ __device__ void decode_item(const MixDecodeArgs& a, const MixItem& it, unsigned 
     r.reserved = 0;
     a.results[it.index] = r;
     *err = 0;
+    *every = 0;
   }
+  return false;
 }
 
 __global__ void __launch_bounds__(kMixThreads, 1) mix_decode_kernel(const __grid_constant__ MixDecodeArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ long long s_item[kMixMaxSlots];
-  __shared__ int s_flag[kMixMaxSlots];
+  __shared__ int s_flag[kMixMaxSlots][2];
   __shared__ unsigned int s_err[kMixMaxSlots];
   const int tid = threadIdx.x;
   if (tid < kMixMaxSlots) {
-    s_flag[tid] = 0;
+    s_flag[tid][0] = s_flag[tid][1] = 0;
     s_err[tid] = 0;
   }
   __syncthreads();
@@ -252,9 +272,12 @@ __global__ void __launch_bounds__(kMixThreads, 1) mix_decode_kernel(const __grid
         slot_sync(bar, nt);
         if (i >= cls.count) break;
         const MixItem it = a.items[cls.first + i];
-        if (cls.straight) decode_item<0>(a, it, sm, cls.max_ncol, st, lt, nt, bar, &s_flag[slot], &s_err[slot]);
-        else if (cls.rows_per_thread == 1) decode_item<1>(a, it, sm, cls.max_ncol, st, lt, nt, bar, &s_flag[slot], &s_err[slot]);
-        else decode_item<2>(a, it, sm, cls.max_ncol, st, lt, nt, bar, &s_flag[slot], &s_err[slot]);
+        bool again;
+        do {
+          if (cls.straight) again = decode_item<0>(a, it, sm, cls.max_ncol, st, lt, nt, bar, s_flag[slot], &s_err[slot]);
+          else if (cls.rows_per_thread == 1) again = decode_item<1>(a, it, sm, cls.max_ncol, st, lt, nt, bar, s_flag[slot], &s_err[slot]);
+          else again = decode_item<2>(a, it, sm, cls.max_ncol, st, lt, nt, bar, s_flag[slot], &s_err[slot]);
+        } while (again);
       }
     }
     __syncthreads();

@@ -33,7 +33,8 @@
 // other row) send the other variables zero while their offsets are not negative, which
 // learned_live_kernel tests before each pass over the frames.  Such a row is then only what
 // it makes of its own column, m the smallest |post| of its other variables:
-//   post_own = s max(alpha m - beta, 0),
+//   post_own = s max(alpha m - beta, 0)
+// (a frame whose magnitudes approach infinity runs again with every row, beyond_skipping),
 // and backward the gradient of post_own's own loss, through alpha m, onto m's variable.  Its
 // record is m, m's variable and two signs.  (Half of base graph 1's rows at rate 1/2, three
 // quarters of base graph 2's: 61 % of its edges.)
@@ -312,17 +313,18 @@ __device__ __forceinline__ void own_column_fwd(const LearnedArgs& a, float* post
 }
 
 // *live: the rows that a pass with shared weights runs: c.rows_live, or all when a skipped row
-// has a negative offset on another edge than its own column's
+// has a negative offset on another edge than its own column's, or there weights that could make
+// a magnitude below beyond_skipping's bound infinite
 __global__ void __launch_bounds__(256) learned_live_kernel(const __grid_constant__ LearnedArgs a) {
   const cbd::DevCode& c = a.code;
   const int first = c.layer_start[c.rows_live], count = c.n_entries - first;
   int bad = 0;
   for (int i = threadIdx.x; i < a.T * count; i += blockDim.x) {
     const int t = i / count, e = first + i - t * count;
-    if (!(a.beta[(size_t)t * c.n_entries + e] < 0.f)) continue;
+    const size_t w = (size_t)t * c.n_entries + e;
     bool own = false;
     for (int L = c.rows_live; L < c.rows_n; L++) own = own || e + 1 == c.layer_start[L + 1];
-    if (!own) bad = 1;
+    if (own ? !cbd::skippable_own_weights(a.alpha[w], a.beta[w]) : a.beta[w] < 0.f) bad = 1;
   }
   bad = __syncthreads_or(bad);
   if (threadIdx.x == 0) *a.live = bad ? c.rows_n : c.rows_live;
@@ -365,32 +367,45 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
   float* post = reinterpret_cast<float*>(smem);
   float2* wbuf = reinterpret_cast<float2*>(smem + learned_post_bytes(c.n_full));  // two iterations' (shared)
   __shared__ float s_loss;
+  __shared__ int s_wide;  // the frame left the magnitudes in which rows may be skipped
   const long long f = blockIdx.x;
   if (f >= a.n_frames) return;
-  if (tid == 0) s_loss = 0.f;
+  if (tid == 0) {
+    s_loss = 0.f;
+    s_wide = 0;
+  }
+  int live = SHARED ? *a.live : c.rows_n;
   unsigned char* tape = a.tape + (size_t)f * a.tape_frame;
   const float* llr = a.llr + (size_t)f * c.e;
+again:
   for (int v = tid; v < c.n_full; v += nt) post[v] = 0.f;
   __syncthreads();
+  Widest<float> widest;
+  auto put = [&](int v, float l) {
+    const float x = __fadd_rn(0.f, l);
+    if constexpr (SHARED) widest.add(x);
+    post[v] = x;
+  };
   if (c.map_is_offset) {
-    for (int t = tid; t < c.e; t += nt) post[2 * z + t] = __fadd_rn(0.f, llr[t]);
+    for (int t = tid; t < c.e; t += nt) put(2 * z + t, llr[t]);
   } else if (!c.has_repeats) {
-    for (int t = tid; t < c.e; t += nt) post[c.map[t]] = __fadd_rn(0.f, llr[t]);
+    for (int t = tid; t < c.e; t += nt) put(c.map[t], llr[t]);
   } else {
     for (int v = tid; v < c.n_full; v += nt) {
       int b0 = c.inv_start[v], b1 = c.inv_start[v + 1];
       if (b0 == b1) continue;
       float s = 0.f;
       for (int i = b0; i < b1; i++) s = __fadd_rn(s, llr[c.inv_t[i]]);
-      post[v] = s;
+      put(v, s);
     }
   }
+  if (SHARED && widest.beyond()) s_wide = 1;
   __syncthreads();
   for (int v = c.k_info + tid; v < c.k; v += nt) post[v] = cbd::kKnownBitLlr;
   __syncthreads();
   const bool multi = a.multi_loss && a.P && a.cw_bits && a.loss;
   const bool active = tid < z;
-  const int live = SHARED ? *a.live : c.rows_n, run = live < c.rows_n ? c.rows_run : c.rows_n;
+  const int run = live < c.rows_n ? c.rows_run : c.rows_n;
   float lsum = 0.f;  // this thread's share of the loss
   // before the first iteration there are no messages: weights that make them 0
   RowWeights<SHARED> wp, wc;
@@ -404,6 +419,11 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
     wp = wc;
     wc = iteration_weights<SHARED>(a, wbuf + (t & 1) * ne, t);
     __syncthreads();
+    if (SHARED && live < c.rows_n && s_wide) {
+      live = c.rows_n;
+      __syncthreads();
+      goto again;
+    }
     const Tape old(tape + (t > 0 ? (size_t)(t - 1) * a.tape_iter : 0), lifted);
     const Tape cur(tape + (size_t)t * a.tape_iter, lifted);
     // the next row's old record is loaded a row ahead
@@ -437,6 +457,7 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
       om = omn;
       if (c.level_end[q]) __syncthreads();
     }
+    if (SHARED && live < c.rows_n && active && beyond_skipping(post, tid, z, c.bg)) s_wide = 1;
     // the skipped rows' own columns, where the loss or the output reads them
     if (SHARED && live < c.rows_n && (t == a.T - 1 || (multi && a.loss_bits > (c.cols_k + live) * z))) {
       if (active) {
@@ -463,6 +484,7 @@ __global__ void __launch_bounds__(384, 2) learned_forward_kernel(const __grid_co
     }
   }
   // outputs
+  if (SHARED && tid == 0) a.frame_live[f] = live;
   if (a.post_out)
     for (int v = tid; v < c.n_full; v += nt) a.post_out[(size_t)f * c.n_full + v] = post[v];
   if (a.cw_bits && a.loss) {
@@ -553,7 +575,7 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
   const int wpc = (c.n_full + 31) >> 5;
   const bool multi = a.multi_loss && a.P;
   const bool active = tid < z;
-  const int live = SHARED ? *a.live : c.rows_n, run = live < c.rows_n ? c.rows_run : c.rows_n;
+  const int live = SHARED ? a.frame_live[f] : c.rows_n, run = live < c.rows_n ? c.rows_run : c.rows_n;
   const bool own_loss = live < c.rows_n && a.loss_bits > (c.cols_k + live) * z;  // on a skipped row's column
   const float scale = 1.f / ((float)a.loss_bits * (float)a.n_frames);
   for (int v = tid; v < c.n_full; v += nt) gp[v] = 0.f;
