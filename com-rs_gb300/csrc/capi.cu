@@ -45,6 +45,7 @@ struct cb_code {
   int32_t* d_inv_t = nullptr;
   void* d_state = nullptr;
   int decode_grid = 0;
+  int sms = 0;              // of the device, once it was used
   unsigned long long* d_counter = nullptr;
   int32_t* d_status = nullptr;
   cudaStream_t stream = nullptr;
@@ -191,7 +192,7 @@ cb_status decode_device_impl(cb_code* c, const T* llr, int64_t n, uint32_t* bits
   a.work_counter = reinterpret_cast<int32_t*>(c->d_counter);
   a.status = c->d_status;
   CB_CUDA(c, cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned long long), s));
-  a.full_grid = c->decode_grid;
+  a.sms = c->sms;
   int grid = (int)std::min<int64_t>(c->decode_grid, n);
   CB_CUDA(c, cbk::launch_decode<T>(a, grid, s));
   return CB_OK;
@@ -535,6 +536,7 @@ cb_status ensure_device(cb_code* c) {
   }
   if (!c->use_nr) c->decode_grid = cbk::decode_grid_size(v, c->precision, c->device);
   if (c->decode_grid <= 0) return fail(c, CB_ERR_CUDA, "the decoder does not fit an SM (occupancy 0)");
+  CB_CUDA(c, cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device));
   CB_CUDA(c, cudaMalloc(&c->d_state, cbk::decode_state_bytes_per_slot(v, c->precision) * c->decode_grid));
   c->dev_ready = true;
   return CB_OK;
@@ -1348,6 +1350,7 @@ cb_status decode_noalloc_impl(cb_code* c, void* scratch, const T* llr, int64_t n
   // once per code object: the occupancy query, and the load of the builds that this and
   // other codes may take, so that no later call maps device memory for one
   if (c->noalloc_grid <= 0 && !use_nr) CB_CUDA(c, cbk::decode_load(c->precision));
+  if (c->sms <= 0) CB_CUDA(c, cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device));
   if (c->noalloc_grid <= 0)
     c->noalloc_grid = use_nr ? cbk::nr_grid_size(k, c->host, c->device)
                              : cbk::decode_grid_size(c->dev, c->precision, c->device);
@@ -1374,7 +1377,7 @@ cb_status decode_noalloc_impl(cb_code* c, void* scratch, const T* llr, int64_t n
     return CB_OK;
   }
   cbk::DecodeArgs<T> a;
-  a.full_grid = occupancy;
+  a.sms = c->sms;
   a.code = c->dev;
   a.cfg = c->cfg;
   a.llr = llr;

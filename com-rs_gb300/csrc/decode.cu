@@ -56,8 +56,9 @@ __host__ __device__ __forceinline__ size_t decode_smem_bytes(int n_full, int z, 
 enum LearnedWeights { kPlain = 0, kWeightsGlobal = 1, kWeightsParam = 2, kWeightsShared = 3 };
 
 // One layered iteration of decode_body: the rows in schedule order, each row's state from
-// the previous iteration (L2-resident), a barrier after each level.  The full f64 build loads
-// the next row's state before the row's update (4096 frames of BG2 Z = 52: 2.80 -> 2.76 ms).
+// the previous iteration (L2-resident), a barrier after each level.  In f64 the next row's
+// state is loaded before the row's update (4096 frames of BG2 Z = 52: 2.80 -> 2.76 ms;
+// base graph 1 0-2 %).
 template <typename T, int LW, int RULE, int MAXD, bool FULL>
 __device__ __forceinline__ void decode_layers(const cbd::DevCode& c, T* post, const StateSlot<T>& st,
                                               const LearnedRowW& lw, int iter, int tid, int z, bool active,
@@ -88,7 +89,7 @@ __device__ __forceinline__ void decode_layers(const cbd::DevCode& c, T* post, co
         row_dispatch_lean<RULE>(d, post, EdgeAddrTable{c.eaddr + s0, tid, 4 * tid, 4 * z}, a1, a2, mt, alpha, n1, n2,
                                 nm);
       else
-        row_dispatch<RULE, MAXD, FULL>(d, post, c.entry + s0, tid, z, a1, a2, mt, scale, n1, n2, nm);
+        row_dispatch<RULE, MAXD, FULL && MAXD == 10>(d, post, c.entry + s0, tid, z, a1, a2, mt, scale, n1, n2, nm);
       st.store(L * z + tid, n1, n2, nm);
     }
     if (c.level_end[q]) __syncthreads();
@@ -112,13 +113,11 @@ __device__ __forceinline__ void row_positions(int (&off)[D], const cbd::DevCode&
 }
 
 // One layered iteration of the f64 decoder with the base graph at compile time
-// (layered_nr.cuh has its schedule), for grids that leave an SM few codewords: a row then
+// (layered_nr.cuh has its schedule), for grids that leave an SM few codewords (lone_rows): a row then
 // waits for a chain of loads (its index, its entries' bounds, the entries, its state), of
 // which the posteriors alone are left.  The state is loaded a row ahead (152 codewords of
 // BG2 Z = 52, generator and decoder: 0.486 ms by decode_layers, 0.448 with the state loaded
-// at its use, 0.42 to 0.44 ahead; 96 words of BG2 Z = 304 from host memory 0.46 -> 0.42).  A
-// full device gains nothing at BG2 Z = 52 and loses at BG1 Z = 64 (2000 codewords 3.57 ->
-// 4.18 ms), so it keeps decode_layers.
+// at its use, 0.42 to 0.44 ahead; 96 words of BG2 Z = 304 from host memory 0.46 -> 0.42).
 template <int BG, int RULE, int Q>
 __device__ __forceinline__ void decode_rows(const cbd::DevCode& c, double* post, const StateSlot<double>& st,
                                             bool first, int r, int z, bool active, const ScaleF64& scale, int live,
@@ -382,17 +381,34 @@ __global__ void __launch_bounds__(384, 2) layered_learned_param_kernel(const __g
   decode_body<float, kWeightsParam, 19, true>(a.d, a.alpha, a.beta);
 }
 
-// The plain decoder.  f64 has four builds: per base graph (2, with rows of at most 10 edges,
-// takes fewer registers), and by whether every SM has its CTAs.  If so, the FP64 pipe bounds
-// the rows: the scaling's products on the integer pipes, the next row's state loaded ahead
-// (4096 codewords of BG2 Z = 52: 8 % less time).  If not, the latency of a row does:
-// decode_rows, and the scaling as two multiplications (on the integer pipes 96 codewords of
-// BG2 Z = 304 take 1-3 % longer).
-void* plain_kernel(int precision, int bg, bool full) {
+// The plain decoder.  f64 has two builds per base graph (2, with rows of at most 10 edges, takes
+// fewer registers): `lone`, decode_rows, and decode_layers with the state loaded ahead and, in
+// base graph 2, the scaling's products on the integer pipes (in base graph 1, whose
+// registers hold an SM at 12 warps, they lose 3-13 % at Z <= 32 and 5 % at Z = 208).
+void* plain_kernel(int precision, int bg, bool lone) {
   if (precision == 1) return (void*)layered_kernel<float, kPlain, 19, true>;
   if (bg == 2)
-    return full ? (void*)layered_kernel<double, kPlain, 10, true> : (void*)layered_kernel<double, kPlain, 10, false>;
-  return full ? (void*)layered_kernel<double, kPlain, 19, true> : (void*)layered_kernel<double, kPlain, 19, false>;
+    return lone ? (void*)layered_kernel<double, kPlain, 10, false> : (void*)layered_kernel<double, kPlain, 10, true>;
+  return lone ? (void*)layered_kernel<double, kPlain, 19, false> : (void*)layered_kernel<double, kPlain, 19, true>;
+}
+
+// Whether a grid of f64 CTAs takes the build for few codewords.  Straight-line rows need each CTA's
+// code to stay in the instruction caches, and gain while a row's latency bounds them.
+// Against decode_layers, every column sent (above 1: faster):
+// Base graph 2, until an SM has the 16 warps that its registers hold and the FP64 pipe bounds
+// it: Z = 52 on 4 / 8 CTAs an SM (8 / 16 warps) 1.20 / 0.90, Z = 208 on 14 warps 1.02, Z = 384 on
+// 12 1.10.
+// Base graph 1, whose registers hold 12 warps: two CTAs an SM (Z = 64 1.05, Z = 208 1.14; one of
+// Z = 384 1.11), and three while each has one codeword (Z = 32 1.05, Z = 64 1.06 to 1.14, Z = 112
+// and 128 1.04; not of three warps, uneven over the four schedulers: Z = 96 0.92, Z = 88 0.99),
+// with half a warp four (Z = 16 1.04).  CTAs that go on to
+// further codewords, or are more, drift apart in the code: Z = 128 on 3 with more codewords
+// 0.97, Z = 64 on 5 0.81, and the times of equal runs on 4 scatter (Z = 64 0.82 to 1.09).
+bool lone_rows(const cbd::DevCode& c, int64_t n_frames, int grid, int sms) {
+  if (sms <= 0) return false;
+  const int per_sm = (grid + sms - 1) / sms, warps = (c.z + 31) / 32;
+  if (c.bg == 2) return per_sm * warps < 16;
+  return per_sm <= 2 || (n_frames <= grid && warps != 3 && per_sm <= (c.z <= 16 ? 4 : 3));
 }
 
 template <typename T>
@@ -400,7 +416,7 @@ void* kernel_for(const DecodeArgs<T>& a, int grid) {
   if constexpr (sizeof(T) == 4) {
     if (a.l_alpha) return a.l_smem ? (void*)layered_kernel<T, kWeightsShared, 19, true> : (void*)layered_kernel<T, kWeightsGlobal, 19, true>;
   }
-  return plain_kernel(sizeof(T) == 8 ? 0 : 1, a.code.bg, grid >= a.full_grid);
+  return plain_kernel(sizeof(T) == 8 ? 0 : 1, a.code.bg, lone_rows(a.code, a.n_frames, grid, a.sms));
 }
 
 int block_threads(int z) { return ((z + 31) / 32) * 32; }
@@ -418,7 +434,7 @@ size_t decode_state_bytes_per_slot(const cbd::DevCode& c, int precision) {
 }
 
 int decode_grid_size(const cbd::DevCode& c, int precision, int device) {
-  void* k = plain_kernel(precision, c.bg, true);
+  void* k = plain_kernel(precision, c.bg, false);
   size_t smem = smem_bytes(c, precision);
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0, sms = 0;

@@ -31,11 +31,11 @@ struct EntryAt {
 // 42.4 against 36.9 ms per 2048 codewords, 3.9 against 3.3 FP64 instructions per edge
 // update).  Only the two additions per edge are left on the FP64 pipe: the posteriors and
 // messages are never -0.0 or NaN, so `l < 0` is the sign bit and the order of non-negative
-// doubles is that of their bit patterns, and with FULL the normalised rule's products are formed by
+// doubles is that of their bit patterns, and with INTS the normalised rule's products are formed by
 // scaled() (4096 frames of BG2 Z = 52 at 9.7 iterations: 3.00 -> 2.80 ms; the pipe 71 % busy,
 // where a kernel of additions alone reaches 84 %).
 // `at` gives the position in post of edge e's variable.
-template <int D, int RULE, bool FULL, typename At>
+template <int D, int RULE, bool INTS, typename At>
 __device__ __forceinline__ void row_update(double* __restrict__ post, const At& at, double a1, double a2, uint32_t mt,
                                            const ScaleF64& scale, double& n1, double& n2, uint32_t& nm) {
   int off[D];
@@ -67,8 +67,8 @@ __device__ __forceinline__ void row_update(double* __restrict__ post, const At& 
   }
   const double m1 = __longlong_as_double(b1), m2 = __longlong_as_double(b2);
   if constexpr (RULE == cbd::RULE_NMS) {
-    n1 = FULL ? scaled(scale, m1) : mul_rn(scale.alpha, m1);
-    n2 = FULL ? scaled(scale, m2) : mul_rn(scale.alpha, m2);
+    n1 = INTS ? scaled(scale, m1) : mul_rn(scale.alpha, m1);
+    n2 = INTS ? scaled(scale, m2) : mul_rn(scale.alpha, m2);
   } else {
     n1 = fmax(sub_rn(m1, scale.alpha), 0.0);
     n2 = fmax(sub_rn(m2, scale.alpha), 0.0);
@@ -270,21 +270,21 @@ __device__ __forceinline__ void row_dispatch_lean(int d, float* post, const Addr
 }
 
 // the row update of the f64 decoder (f32 rows take row_dispatch_lean); rows of at most MAXD edges
-template <int RULE, int MAXD, bool FULL>
+template <int RULE, int MAXD, bool INTS>
 __device__ __forceinline__ void row_dispatch(int d, double* post, const uint32_t* ent, int r, int z, double a1,
                                              double a2, uint32_t mt, const ScaleF64& scale, double& n1, double& n2,
                                              uint32_t& nm) {
   switch (d) {
-    case 3: row_update<3, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
-    case 4: row_update<4, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
-    case 5: row_update<5, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
-    case 6: row_update<6, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
-    case 7: row_update<7, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
-    case 8: row_update<8, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
-    case 9: row_update<9, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
-    case 10: row_update<10, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 3: row_update<3, RULE, INTS>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 4: row_update<4, RULE, INTS>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 5: row_update<5, RULE, INTS>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 6: row_update<6, RULE, INTS>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 7: row_update<7, RULE, INTS>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 8: row_update<8, RULE, INTS>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 9: row_update<9, RULE, INTS>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
+    case 10: row_update<10, RULE, INTS>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm); break;
     default:
-      if constexpr (MAXD > 10) row_update<19, RULE, FULL>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm);
+      if constexpr (MAXD > 10) row_update<19, RULE, INTS>(post, EntryAt{ent, r, z}, a1, a2, mt, scale, n1, n2, nm);
       break;
   }
 }

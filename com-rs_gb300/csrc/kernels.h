@@ -30,7 +30,7 @@ struct DecodeArgs {
   const float* l_beta = nullptr;
   int32_t l_shared = 0;
   int32_t l_smem = 0;  // 1: each iteration's (shared) weights staged in shared memory
-  int32_t full_grid = 0;  // f64: the resident CTAs that fill the device (0: not known, taken as full)
+  int32_t sms = 0;  // f64: the device's SMs (0: not known)
 };
 
 // The learned decoder with its weights in the launch parameters (weights shared across

@@ -50,3 +50,17 @@ def test_no_alloc_calls_after_the_first_map_no_kernel(cb):
         assert L.cb_decode_device(gen._h, ptr(llr), len(llr), ptr(out[1]), None, ptr(its[1]), stream) == 0
         torch.cuda.synchronize()
         assert torch.equal(out[0], out[1]) and torch.equal(its[0], its[1])
+
+
+@pytest.mark.parametrize("bg, z, per_sm", [(1, 32, (3, 4)), (1, 64, (3, 4)), (1, 96, (2, 3)), (1, 120, (3, 4)),
+                                           (2, 20, (15, 16)), (2, 52, (7, 8)), (2, 128, (3, 4)), (2, 208, (2, 3))])
+def test_the_builds_agree_at_the_line_between_them(cb, bg, z, per_sm):
+    # codeword counts on both sides of the CTAs per SM at which the build changes
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    k, cols = (22 if bg == 1 else 10) * z, 66 if bg == 1 else 50
+    g = cb.NrLdpc(k, cols * z, base_graph=bg, lifting_size=z, precision="f64", max_iterations=6)
+    runs = [g.run_frames(3, "line", 0, 0, p * sms + d, 0.0, 4) for p in per_sm for d in (0, 1)]
+    for r in runs[:-1]:
+        assert np.array_equal(r, runs[-1][:len(r)])
