@@ -263,10 +263,11 @@ __device__ __forceinline__ void gen_one(const cbd::DevCode& c, const GenFrame<T>
   }
 }
 
-// (f32: five CTAs on an SM, 96 registers; f64: four, 128: the FP64 work of one covers the jumps, the encoding
-// and the power sum of the others; 4096 BG2 Z = 52 QPSK frames 1.30 -> 1.22 ms)
-template <typename T>
-__global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 4 : 5) gen_kernel(const __grid_constant__ GenArgs<T> a) {
+// CTAS on an SM.  f32: five, 96 registers; f64: four, 128: the FP64 work of one covers the jumps, the encoding
+// and the power sum of the others; 4096 BG2 Z = 52 QPSK frames 1.30 -> 1.22 ms.  (f64 with three,
+// 168 registers: see many_points.)
+template <typename T, int CTAS>
+__global__ void __launch_bounds__(NT, CTAS) gen_kernel(const __grid_constant__ GenArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const long long frame = (long long)blockIdx.x;
   if (frame >= a.n_frames) return;
@@ -331,10 +332,30 @@ size_t gen_smem_bytes(const cbd::DevCode& c, int m, int mbits, int n_pad) {
   return (size_t)2 * m * sizeof(double) + (size_t)(ncol + 4) * ws * 4 + c.n_full + n_sym + 16;
 }
 
+namespace {
+// Whether the frames spend their time in the exact demapper of 256 points, which alone keeps the
+// FP64 pipe busy and loses 3-4 % to the spills of 128 registers: frames of at least a symbol
+// a thread, in several rounds of three CTAs an SM.  4096 frames of BG2 Z = 52 121 against 117 ms,
+// 2048 of BG1 Z = 64 133 against 129; 8192 of 20 symbols (BG2 Z = 8) 40 against 44, 512 of
+// BG1 Z = 384, whose 3.4 CTAs an SM are one round of four, 184 against 285.
+bool many_points(const GenArgs<double>& a) {
+  if (!a.exact || a.m != 256 || (a.code.e + a.n_pad) / a.mbits < NT) return false;
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+    return false;
+  return a.n_frames > (int64_t)12 * sms;
+}
+void* gen_kernel_ptr(const GenArgs<double>& a) {
+  return many_points(a) ? (void*)gen_kernel<double, 3> : (void*)gen_kernel<double, 4>;
+}
+void* gen_kernel_ptr(const GenArgs<float>&) { return (void*)gen_kernel<float, 5>; }
+}  // namespace
+
 template <typename T>
 cudaError_t launch_gen(const GenArgs<T>& a, cudaStream_t stream) {
   size_t smem = gen_smem_bytes(a.code, a.m, a.mbits, a.n_pad);
-  void* k = (void*)gen_kernel<T>;
+  void* k = gen_kernel_ptr(a);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void* args[] = {(void*)&a};
