@@ -15,7 +15,7 @@
 // Measured (GB300, f64, words with the copies): PEG(1024, 512), 4096 words of 13 iterations
 // 69 -> 30 ms; PEG(576, 288), 2000 words of 3 iterations, some of 50, 16.9 -> 5.1 ms; one
 // word of PEG(301, 150) 0.87 -> 0.23 ms.  f32 1.3-1.9 times faster.  What is left is the
-// FP64 pipe, 75-80 % busy: about 67 instructions an edge (tanh 14 or 24, atanh 36).
+// FP64 pipe, 81-85 % busy.
 // The product is formed as check_row (sparse.cu) forms it: the running product of the
 // edges before, first to last, times that of the edges after, last to first, so the results
 // are the same bits.
@@ -29,10 +29,12 @@ namespace {
 
 __device__ __forceinline__ void slot_sync(int bar, int n) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory"); }
 
-// The high word of the |l| (1.31) near which CUDA's f64 tanh(l / 2) changes its method, found by
-// counting its FP64 instructions (14 below, 24 above): the edges of a level are ordered by
-// it, so that a warp runs one method and not both (38).  It only orders the work.
-constexpr int kTanhSplitHi = 0x3ff4f5c3;
+// The edges of a level are grouped by the size of |l|, so that the lanes of a warp have arguments of
+// one kind: it orders the work and nothing else.  The high word of 5/4, the fastest of six round
+// values for the whole decode: the link of 512 trials 33.5 ms, with 1/2 37.5, 1 36.5, 3/2 35.3,
+// 2 35.8, 3 36.5 and one group 36.7; PEG(576, 288), 2000 words 4.13 (4.41, 4.28, 4.39, 4.63, 4.61,
+// 4.23).
+constexpr int kGroupSplitHi = 0x3ff40000;
 
 // x / 2, for doubles by the exponent field (off the FP64 pipe) unless the result could be
 // subnormal or x is not finite
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(kEdgeThreads, 1) sparse_edges_kernel(const __g
                 const int v = (int)(edge[e] & 0xffffu);
                 const T l = sub_rn(post[v], msg[e]);
                 post[v] = l;
-                small = (__double2hiint(l) & 0x7fffffff) < kTanhSplitHi;
+                small = (__double2hiint(l) & 0x7fffffff) < kGroupSplitHi;
               }
               const unsigned ms = __ballot_sync(0xffffffffu, in && small), ml = __ballot_sync(0xffffffffu, in && !small);
               int at = 0;
