@@ -1,5 +1,6 @@
 // The C ABI of include/comrs_gb300.h: code objects, device buffers, chunked launches.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -69,6 +70,7 @@ struct cb_code {
   uint8_t* d_u8 = nullptr;  // the encoder's information and sent bytes
   size_t u8_cap = 0;
   int encode_on = 0;        // where blocks are encoded: 0 not yet known, 1 the device, 2 the host
+  pid_t encode_pid = 0;     // the process in which that was found
   std::vector<uint32_t> h_words;
   std::map<int, GenCache> gen;
   bool dev_ready = false;
@@ -437,7 +439,12 @@ cudaError_t ensure_map(cb_code* c) {
   return cudaSuccess;
 }
 
-// The blocks through the encoding kernel, in chunks whose bytes stay within 256 MB.
+// Bytes of a chunk in the encoder's device buffer, which the code object keeps (grow may make
+// it half as large again).  A chunk costs some 40 us beside its copies: 14,000 blocks of
+// BG1 Z = 384, 474 MB, take 3.24 ms in chunks of 256 MB, 3.77 of 32.
+constexpr size_t kEncodeBytes = (size_t)128 << 20;
+
+// The blocks through the encoding kernel, in chunks of kEncodeBytes.
 // Only the stream and the rate matching's map are set up: encoding needs no decoder.  The
 // caller's current device stays what it was, and a stream capture of the calling thread
 // goes on undisturbed (the relaxed mode allows the allocations made here).
@@ -459,7 +466,7 @@ cudaError_t encode_device(cb_code* c, const uint8_t* info, int64_t n, uint8_t* o
   if (e == cudaSuccess && !c->stream) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = ensure_map(c);
   const size_t per = (size_t)h.k_info + h.e;
-  const int64_t chunk = std::min<int64_t>(n, std::max<int64_t>(1, (int64_t)(((size_t)256 << 20) / per)));
+  const int64_t chunk = std::min<int64_t>(n, std::max<int64_t>(1, (int64_t)(kEncodeBytes / per)));
   // the sent bytes first: their rows are 4-byte aligned when E is a multiple of 4
   if (e == cudaSuccess) e = grow(c->d_u8, c->u8_cap, (size_t)chunk * per);
   *ready = e == cudaSuccess;
@@ -476,8 +483,9 @@ cudaError_t encode_device(cb_code* c, const uint8_t* info, int64_t n, uint8_t* o
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(out + (size_t)done * h.e, c->d_u8, (size_t)cnt * h.e, cudaMemcpyDeviceToHost, c->stream);
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  return e;
+  // (after an error too: no copy is left in flight on the caller's buffers)
+  const cudaError_t end = *ready ? cudaStreamSynchronize(c->stream) : cudaSuccess;
+  return e == cudaSuccess ? end : e;
 }
 
 // Work (lifted edges of all blocks) from which the encoder runs on the device: the host
@@ -682,6 +690,8 @@ cb_status cb_encode(cb_code* c, const uint8_t* info, int64_t n, uint8_t* out) {
   if (!c || !info || !out || n < 0) return fail(c, CB_ERR_CONFIG, "NULL argument or negative count");
   std::lock_guard<std::mutex> lock(c->mu);
   const cbh::NrCode& h = c->host;
+  // a process forked after the device was used must not touch it: there the host encodes
+  if (c->encode_on == 1 && c->encode_pid != getpid()) c->encode_on = 2;
   if (c->encode_on != 2 && n * h.edges >= kEncodeDeviceEdges) {
     if (c->encode_on == 0) {
       // a code object encodes on a machine without its GPU too
@@ -691,6 +701,7 @@ cb_status cb_encode(cb_code* c, const uint8_t* info, int64_t n, uint8_t* out) {
         count = 0;
       }
       c->encode_on = c->device >= 0 && c->device < count ? 1 : 2;
+      c->encode_pid = getpid();
     }
     if (c->encode_on == 1) {
       bool ready = false;

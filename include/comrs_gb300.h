@@ -109,7 +109,13 @@ cb_status cb_code_info(const cb_code* code, int64_t info[16]);
  * pointer may be NULL.  Sizes from cb_code_info. */
 cb_status cb_code_tables(const cb_code* code, int32_t* entries, int32_t* bit_map);
 
-/* Encode n_frames blocks: info = n_frames x K' bytes (0/1), out = n_frames x E bytes. */
+/* Encode n_frames blocks: info = n_frames x K' bytes (0/1), out = n_frames x E bytes, both in
+ * host memory.  From 2^15 lifted edges on (n_frames times the edges of cb_code_info) the
+ * blocks are encoded on the code's device; smaller calls, and all on a machine without the
+ * device, on the host, with the same bytes.  The first such call initialises CUDA in the process
+ * and makes a stream and a device buffer of at most 192 MB, kept until cb_code_destroy.  A
+ * process forked from one that has done so encodes on the host, and, as with every use of
+ * CUDA before a fork, cannot use the device itself. */
 cb_status cb_encode(cb_code* code, const uint8_t* info, int64_t n_frames, uint8_t* out);
 
 /* Decode n_frames blocks of E channel LLRs (double for CB_F64, float for CB_F32),
