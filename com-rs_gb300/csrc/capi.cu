@@ -897,7 +897,7 @@ cb_status nms_buffers(cb_nms* h, int64_t n, NmsUse use) {
     CB_CUDA(c, grow(h->d_tape, h->tape_cap, (size_t)n * (use == kNmsTrain ? h->T : 1) * cbk::learned_tape_bytes(c->dev)));
   }
   if (use == kNmsTrain) {
-    CB_CUDA(c, grow(h->d_c2v, h->c2v_cap, (size_t)n * c->dev.n_entries * cbk::learned_stride(c->dev) * 4));
+    CB_CUDA(c, grow(h->d_c2v, h->c2v_cap, (size_t)n * c->dev.n_entries * cbk::learned_stride(c->dev, h->shared) * 4));
     CB_CUDA(c, grow(h->d_P, h->P_cap, (size_t)n * h->T * c->host.n_full * 4));
     CB_CUDA(c, grow(h->d_cw, h->cw_cap, (size_t)n * ((c->host.n_full + 31) / 32) * 4));
     CB_CUDA(c, grow(h->d_ebn0, h->ebn0_cap, (size_t)n * 4));

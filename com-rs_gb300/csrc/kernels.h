@@ -192,9 +192,16 @@ struct LearnedArgs {
   int32_t* live;
   int32_t* frame_live;
 };
-// from one base-graph entry's message gradients to the next's: a compile-time constant of
-// the backward kernels
-inline int learned_stride(const cbd::DevCode& c) { return c.z <= 64 ? 64 : 384; }
+// From one base-graph entry's message gradients to the next's.  Shared weights: a compile-time
+// constant of the backward kernel, less than twice Z from 16 on (with 64 and 384 alone a frame of
+// Z = 66 took 5.8 times what its edges need; with Z itself, not a constant, 1024 frames' step
+// of BG2 Z = 20 to 128 took 8-10 % longer, 304 of BG1 Z = 256 17 %).
+inline int learned_stride(const cbd::DevCode& c, bool shared) {
+  if (!shared) return c.z;
+  for (int s = 16; s <= 256; s *= 2)
+    if (c.z <= s) return s;
+  return 384;
+}
 inline size_t learned_tape_bytes(const cbd::DevCode& c) { return (((size_t)c.rows_n * c.z * 12) + 15) & ~(size_t)15; }
 cudaError_t launch_learned(const LearnedArgs& a, bool forward, cudaStream_t stream);
 // codeword bytes [n_frames][n_bits] to packed words [n_frames][ceil(n_bits / 32)], LSB first

@@ -217,15 +217,16 @@ __device__ __forceinline__ void put_warp_sums(float (&v)[N], float* red, int lan
   }
 }
 
-// Backward of one lifted row from its record.  `gr` points at the row's message gradients,
-// S floats from edge to edge (a constant, so that their addresses are immediates).  With
+// Backward of one lifted row from its record.  `gr` points at the row's message gradients, S
+// floats from edge to edge (a constant, so that their addresses are immediates; 0: z, with weights
+// per lifted edge, whose atomics hide it).  With
 // shared weights `red` receives the warp's sums of the gradients: D scales, then D offsets with the
 // opposite sign (every lane of the warp takes part; the lanes without a row with zeros).
 template <int D, bool SHARED, int S>
 __device__ __forceinline__ void learned_row_bwd(const LearnedArgs& a, float* gp, float* gr, float2 n, uint32_t nm,
                                                 int t, int s0, int r, int z, bool active, bool last,
                                                 const RowWeights<SHARED>& w, float* red, int lane) {
-  const int i1 = (int)(nm & 31u);
+  const int i1 = (int)(nm & 31u), st = S ? S : z;
   float ga[D];  // the gradients of max(alpha m - beta, 0): of the offsets, negated
   if (active) {
     const EdgeAddrTable addr{a.code.eaddr + s0, r, 4 * r, 4 * z};
@@ -233,7 +234,7 @@ __device__ __forceinline__ void learned_row_bwd(const LearnedArgs& a, float* gp,
     int i2 = (int)((nm >> 5) & 31u);
     const uint32_t sg = nm & kMetaSigns, ns = (__popc(sg) & 1) ? ~sg : sg;
 #pragma unroll
-    for (int e = 0; e < D; e++) ga[e] = last ? 0.f : gr[e * S];
+    for (int e = 0; e < D; e++) ga[e] = last ? 0.f : gr[e * st];
     float g1 = 0.f, g2 = 0.f;  // gradients of |x_i1| and |x_i2|
 #pragma unroll
     for (int e = 0; e < D; e++) {
@@ -262,7 +263,7 @@ __device__ __forceinline__ void learned_row_bwd(const LearnedArgs& a, float* gp,
       const bool at1 = e == i1, at2 = e == i2;
       const float gx = ld_post(gp, off[e]) + (at1 ? g1 : at2 ? g2 : 0.f);
       if (at1 || at2) st_post(gp, off[e], gx);
-      if (t > 0) gr[e * S] = -gx;
+      if (t > 0) gr[e * st] = -gx;
     }
   } else {
 #pragma unroll
@@ -571,7 +572,8 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
   constexpr int RW = 2 * kMaxLevelEdges;
   const long long f = blockIdx.x;
   if (f >= a.n_frames) return;
-  float* gc = a.c2v + (size_t)f * c.n_entries * S + tid;  // this thread's message gradients
+  const int st = S ? S : z;
+  float* gc = a.c2v + (size_t)f * c.n_entries * st + tid;  // this thread's message gradients
   const int wpc = (c.n_full + 31) >> 5;
   const bool multi = a.multi_loss && a.P;
   const bool active = tid < z;
@@ -639,7 +641,7 @@ __global__ void __launch_bounds__(384, 2) learned_backward_kernel(const __grid_c
         if (qe > 0) record(qe - 1, nn, nmn);
         float* rd = red + ((size_t)buf * nw + warp) * RW + 2 * at;
 #define CB_ROW(DD)                                                                                                 \
-  learned_row_bwd<DD, SHARED, S>(a, gp, gc + (size_t)s0 * S, n, nm, t, s0, tid, z, active && L < live, t == a.T - 1, w, rd, lane);
+  learned_row_bwd<DD, SHARED, S>(a, gp, gc + (size_t)s0 * st, n, nm, t, s0, tid, z, active && L < live, t == a.T - 1, w, rd, lane);
         CB_LEARNED_DEGREES(CB_ROW)
 #undef CB_ROW
         n = nn;
@@ -704,12 +706,20 @@ cudaError_t launch_learned(const LearnedArgs& a, bool forward, cudaStream_t s) {
   }
   const int threads = ((a.code.z + 31) / 32) * 32;
   void* k;
-  if (forward) {
+  if (!forward && !a.shared) {
+    k = (void*)learned_backward_kernel<false, 0>;
+  } else if (forward) {
     k = a.shared ? (void*)learned_forward_kernel<true> : (void*)learned_forward_kernel<false>;
-  } else if (learned_stride(a.code) == 64) {
-    k = a.shared ? (void*)learned_backward_kernel<true, 64> : (void*)learned_backward_kernel<false, 64>;
   } else {
-    k = a.shared ? (void*)learned_backward_kernel<true, 384> : (void*)learned_backward_kernel<false, 384>;
+    switch (learned_stride(a.code, a.shared)) {
+      case 16: k = (void*)learned_backward_kernel<true, 16>; break;
+      case 32: k = (void*)learned_backward_kernel<true, 32>; break;
+      case 64: k = (void*)learned_backward_kernel<true, 64>; break;
+      case 128: k = (void*)learned_backward_kernel<true, 128>; break;
+      case 256: k = (void*)learned_backward_kernel<true, 256>; break;
+      case 384: k = (void*)learned_backward_kernel<true, 384>; break;
+      default: return cudaErrorInvalidValue;
+    }
   }
   size_t smem = learned_post_bytes(a.code.n_full);
   if (a.shared)
