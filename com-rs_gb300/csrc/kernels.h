@@ -150,7 +150,7 @@ struct MixDecodeArgs {
   const cbd::DevCode* codes;
   const MixItem* items;     // sorted by class
   const MixClass* classes;
-  int32_t n_classes, rule, max_it;
+  int32_t n_classes, rule, max_it;  // rule: RULE_NMS
   float alpha;
   const float* llr;
   const uint32_t* info;

@@ -84,7 +84,10 @@ __device__ bool slot_check_fails(const float* post, uint32_t* hd, const uint32_t
 // (layered_nr.cuh), the edge addresses from the slot's table.  Bound by issue: the degree and
 // the entries' bounds are no longer read and branched on per row.  Used for slots of at
 // least 128 threads; 16384 uneven codewords, generator and decoder: 9.32 ms, 9.99 with no
-// slot on it, 9.41 from 256 threads, 9.52 from 64 and 9.70 with all slots on it.
+// slot on it, 9.41 from 256 threads, 9.52 from 64 and 9.70 with all slots on it.  The
+// normalised rule only, the one a batch has.  (The table-driven rows keep the offset rule's
+// branch, which nothing reaches: without it the compiler's registers fall out 1 % worse at 16384
+// codewords and 20 % at 300.)
 struct MixTable {
   const uint2* eaddr;  // {4 shift, 4 column Z} per entry
 };
@@ -303,6 +306,7 @@ int mix_decode_grid(size_t smem, int device) {
 }
 
 cudaError_t launch_mix_decode(const MixDecodeArgs& a, int grid, size_t smem, cudaStream_t s) {
+  if (a.rule != cbd::RULE_NMS) return cudaErrorInvalidValue;  // (mix_rows has no other)
   void* k = (void*)mix_decode_kernel;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
