@@ -30,11 +30,11 @@ namespace {
 __device__ __forceinline__ void slot_sync(int bar, int n) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory"); }
 
 // The edges of a level are grouped by the size of |l|, so that the lanes of a warp have arguments of
-// one kind: it orders the work and nothing else.  The high word of 5/4, the fastest of six round
-// values for the whole decode: the link of 512 trials 33.5 ms, with 1/2 37.5, 1 36.5, 3/2 35.3,
-// 2 35.8, 3 36.5 and one group 36.7; PEG(576, 288), 2000 words 4.13 (4.41, 4.28, 4.39, 4.63, 4.61,
-// 4.23).
-constexpr int kGroupSplitHi = 0x3ff40000;
+// one kind: it orders the work and nothing else.  The high word of 21/16, the fastest value of
+// those tried (sixteenths from 18 to 24, and 1/2, 1, 2 and 3) by the time of the whole decode:
+// the link of 512 trials at 2.5 dB 91 ms, with 20/16 97, 22/16 98, 18/16 103 and 24/16 102; at 4 dB
+// 33.0 ms, 33.6 to 34.1, 34.5, 35.0 and 35.0, with 1 36.5, 3 36.5 and one group 36.7.
+constexpr int kGroupSplitHi = 0x3ff50000;
 
 // x / 2, for doubles by the exponent field (off the FP64 pipe) unless the result could be
 // subnormal or x is not finite
