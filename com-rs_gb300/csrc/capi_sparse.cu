@@ -222,8 +222,8 @@ cb_status ensure_device(cb_ldpc* c) {
     if (use_chain(c, blocks)) return ensure_chain(c, blocks);
   }
   // sum-product levels of more than eight rows whose word fits shared memory: an edge per
-  // thread, in f64 (1.8-3.7 times faster than a thread per row, sparse_edges.cu) and in f32
-  // (1.2-1.8 times).  Levels of fewer rows keep the warp per row, which associates the
+  // thread, in f64 (1.3-4.3 times faster than a thread per row, sparse_edges.cu) and in f32
+  // (1.0-2.2 times).  Levels of fewer rows keep the warp per row, which associates the
   // products as a scan does.
   c->edge_slots = 0;
   if (c->layered && c->rule == CB_RULE_SUM_PRODUCT && h.max_level_rows > 8) {

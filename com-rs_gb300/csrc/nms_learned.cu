@@ -42,7 +42,7 @@
 // Bound: forward, issue (57-65 %); backward, the latency of the message gradients, 4 bytes
 // an edge read and written per iteration, more than L2 holds for BG1's resident frames.
 // Measured on GB300, shared weights: a step of 512 frames of BG1 Z = 384, 8 iterations, 10.3
-// -> 3.2 ms (forward 3.57, backward 6.52 before; 1.43 and 2.15 with every row run); 1024
+// -> 3.3 ms (forward 3.57, backward 6.52 before; 1.43 and 2.15 with every row run); 1024
 // frames of BG2 Z = 52, 10 iterations, forward 0.98 -> 0.36 ms (0.46 with every row) and
 // backward 1.78 -> 0.44 (0.67).  Before: x on the tape, messages and weights read from global memory
 // in the rows, ten shuffles per edge for the weight gradients and their sums by shared-memory

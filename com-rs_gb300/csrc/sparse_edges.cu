@@ -12,10 +12,10 @@
 //   * the edges of a level are spread over the slot's lanes: each computes its tanh, then,
 //     after a barrier, the product of the row's other tanh values and its own outgoing
 //     message.
-// Measured (GB300, f64, words with the copies): PEG(1024, 512), 4096 words of 13 iterations
-// 69 -> 30 ms; PEG(576, 288), 2000 words of 3 iterations, some of 50, 16.9 -> 5.1 ms; one
-// word of PEG(301, 150) 0.87 -> 0.23 ms.  f32 1.3-1.9 times faster.  What is left is the
-// FP64 pipe, 81-85 % busy.
+// Measured (GB300, words with the copies): the link of 512 trials, 4096 words of PEG(1024, 512),
+// 76.7 -> 33.0 ms; PEG(576, 288), 2000 words of 3 iterations, some of 50, 20.7 -> 5.6 ms
+// (15.3 -> 4.6 on another box).  PEG codes of 301 to 4000 bits, 1 to 3000 words: f64 1.3 to
+// 4.3 times faster, f32 1.0 to 2.2.  What is left in f64 is the FP64 pipe, 81-85 % busy.
 // The product is formed as check_row (sparse.cu) forms it: the running product of the
 // edges before, first to last, times that of the edges after, last to first, so the results
 // are the same bits.

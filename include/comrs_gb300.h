@@ -123,7 +123,11 @@ cb_status cb_encode(cb_code* code, const uint8_t* info, int64_t n_frames, uint8_
  * app: n_frames x K' a posteriori LLRs of the information bits (optional);
  * iterations: n_frames int32 (optional).  Page-locked LLRs (cudaHostAlloc,
  * cudaHostRegister) are read by the decoder in place; others are copied to the device in
- * chunks that overlap the decoding.  The results are the same. */
+ * chunks that overlap the decoding.  The results are the same.
+ * LLRs may be infinite.  The layered min-sum's equality with the reference, bit for bit,
+ * holds while the LLRs and the sums of LLRs and messages are finite: where infinite ones
+ * meet, inf - inf is NaN, and the GPU's minimum search does not order NaN as the
+ * reference's comparisons do. */
 cb_status cb_decode(cb_code* code, const void* llr, int64_t n_frames, uint8_t* bits, void* app,
                     int32_t* iterations);
 
