@@ -76,6 +76,19 @@ def test_edge_parallel_rows_equal_a_thread_per_row(cb, n, m, dmin, dmax, seed, f
     _same(gpu, other, llr, 60000, dt)
 
 
+@pytest.mark.parametrize("precision, dt", PRECISIONS)
+@pytest.mark.parametrize("degree", [255, 256])
+def test_the_longest_rows_of_an_edge_a_thread(cb, degree, precision, dt):
+    # a row of 256 edges leaves the code to the kernel with several words a CTA and a thread a row
+    n = 700
+    rows = [list(range(degree))] + [[degree + 2 * i, degree + 2 * i + 1] for i in range(12)]
+    rows += [sorted(np.random.default_rng(i).choice(n, 5, replace=False).tolist()) for i in range(60)]
+    kw = dict(max_iterations=9, precision=precision, encoder=None)
+    gpu, other = cb.Ldpc(n, rows, **kw), cb.Ldpc(n + 60000, rows, **kw)
+    assert gpu.info()["max_level_rows"] > 8
+    _same(gpu, other, np.random.default_rng(degree).normal(4.0, 2.0, (40, n)), 60000, dt)
+
+
 @pytest.mark.parametrize("kind, shape", [("chain", s) for s in CHAINS] + [("edges", s) for s in EDGES])
 def test_f32_agrees_with_the_oracle_after_one_iteration(cb, O, kind, shape):
     # rows of at least three edges and LLRs within +-3: a message's product of tanh values is wrong

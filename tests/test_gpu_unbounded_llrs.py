@@ -57,6 +57,28 @@ def test_unbounded_words_decode_as_with_every_row(cb, O, bg, z, cols, rule, alph
             assert its[f] == rits[f] and np.array_equal(bits[f], rbits[f]) and same(app[f], rapp[f]), f % len(llr)
 
 
+@pytest.mark.parametrize("precision, powers", [("f64", (0, 900, 997, 1012)), ("f32", (0, 80, 97, 112))])
+@pytest.mark.parametrize("bg, z, cols", CODES)
+def test_large_finite_words_equal_the_oracle(cb, O, bg, z, cols, precision, powers):
+    # the normalised rule commutes with a power of two while nothing overflows: magnitudes below, at
+    # and beyond the bound from which every row runs, and words that pass it while decoding
+    dtype = np.float64 if precision == "f64" else np.float32
+    k, e = (22 if bg == 1 else 10) * z, cols * z
+    g = cb.NrLdpc(k, e, base_graph=bg, lifting_size=z, precision=precision, max_iterations=8)
+    ref = O.Code(k, e, bg=bg, z=z).set_decoder(O.RULE_NMS, 0.75, True, 8)
+    rng = np.random.default_rng(cols)
+    s = 1.0 - 2.0 * np.stack([ref.encode(u) for u in rng.integers(0, 2, (6, k)).astype(np.uint8)])
+    llr = (3.0 * s + 4.0 * rng.standard_normal(s.shape)).astype(dtype)
+    bits, app, its = g.decode_full(np.concatenate([llr * dtype(2.0) ** p for p in powers]))
+    word = np.uint64 if precision == "f64" else np.uint32
+    for i, p in enumerate(powers):
+        for f in range(len(llr)):
+            rb, rit, rapp, _ = ref.decode(llr[f] * dtype(2.0) ** p, precision, want_app=True)
+            at = i * len(llr) + f
+            assert np.all(np.isfinite(rapp)) and rit == its[at], (p, f)
+            assert np.array_equal(rb, bits[at]) and np.array_equal(rapp.view(word), app[at].view(word)), (p, f)
+
+
 @pytest.mark.parametrize("precision", ["f64", "f32"])
 def test_unbounded_words_without_allocation(cb, O, precision):
     import torch
